@@ -202,6 +202,7 @@ mrg_status mrg_destroy(mrg_ctx* c)
     cudaFree(c->ptPathMem2);
     cudaFree(c->dPtRadTotal2);
     cudaFree(c->dPtGradEmission);
+    for(void* q : c->dPtAdjRec) cudaFree(q);
     cudaFree(c->dZsTables);
     cudaFree(c->dZsSeeds);
     cudaFree(c->dHostCounters);

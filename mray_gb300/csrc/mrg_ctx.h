@@ -119,6 +119,8 @@ struct mrg_ctx
     cudaEvent_t  ptEvFilm = nullptr, ptEvStart = nullptr, ptEvDone2 = nullptr;
     void*        dPtRadTotal2 = nullptr;      // adjoint: primal radiance of the second pipeline
     uint32_t     ptRadTotalCap2 = 0;
+    void*        dPtAdjRec[2] = { nullptr, nullptr };   // adjoint: vertex records of each pipeline's pass
+    uint64_t     ptAdjRecCap[2] = { 0, 0 };             // records
     double*      dPtGradEmission = nullptr;   // adjoint: FP64 emission-gradient sums, RGBA per instance
     uint32_t*    dZsTables = nullptr;         // ZSobol sampler: matrices and digit permutations
     uint32_t*    dZsSeeds = nullptr;          // ZSobol sampler: per-pixel seeds of (zsW, zsH, zsSeed)

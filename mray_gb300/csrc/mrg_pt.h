@@ -77,18 +77,35 @@ struct PtSpectral
     uint32_t     enabled;
 };
 
-// Path-replay adjoint of the image with respect to an f32 albedo texture
-// (no reference counterpart): the replay of a pass scatters
+// Adjoint of the image with respect to an f32 albedo texture (no reference
+// counterpart): every Lambert vertex whose albedo is the texture adds
 // delta[pixel] * (radiance after the vertex) / albedo * bilinear weight
-// into grad for every Lambert vertex whose albedo is the texture.
+// into grad.  The radiance after a vertex is known when the path has ended:
+// kAdjRecord keeps a record per such vertex and scatters them after the
+// pass; kAdjReplay walks the pass a second time with the primal radiance.
+enum PtAdjointMode : uint32_t { kAdjOff = 0, kAdjReplay = 1, kAdjRecord = 2 };
+
+// Vertex records of one pass: a = (slot, primitive, barycentrics of the hit),
+// b = (albedo, radiance before .x), c = (radiance before .yz).
+struct PtAdjointRecords
+{
+    uint32_t* count;
+    float4*   a;
+    float4*   b;
+    float2*   c;
+    uint32_t  cap;
+};
+constexpr size_t kAdjRecordBytes = 40;
+
 struct PtAdjoint
 {
     const float4* delta;        // dLoss / dPixel (RGB) per pixel
     float*        grad;         // RGBA per texel (A unused)
-    const float4* radTotal;     // primal radiance per path slot
+    const float4* radTotal;     // kAdjReplay: primal radiance per path slot
+    PtAdjointRecords rec;       // kAdjRecord
     uint32_t      texIndex;     // texture id + 1 (0: no texture parameter)
     float         invSpp;       // 1 / samples per pixel of the image
-    uint32_t      enabled;
+    uint32_t      mode;         // PtAdjointMode
     double*       gradEmission; // RGBA per instance: dLoss / d(area-light radiance), FP64 sums, or null
 };
 
@@ -210,6 +227,9 @@ cudaError_t pt_cache_targets(const PtPaths& P, const PtCacheUse& C, const PtSpec
                              cudaStream_t st);
 cudaError_t pt_resolve(const PtLaunch& L, const PtPaths& P, const PtLight* lights, uint32_t depth, int smCount,
                        cudaStream_t st);
+// The texture gradient of a pass's vertex records (L.adj.rec), after the pass.
+cudaError_t pt_adjoint_scatter(const PtLaunch& L, const PtPaths& P, const PtSceneTables& T, int smCount,
+                               cudaStream_t st);
 // out[i] += acc[i] (f32 from the FP64 emission-gradient sums), n entries.
 cudaError_t pt_add_emission_grad(const double* acc, float* out, uint32_t n, cudaStream_t st);
 cudaError_t pt_film(const PtLaunch& L, const PtPaths& P, float4* image, cudaStream_t st);

@@ -1148,30 +1148,56 @@ __global__ void k_add_emission_grad(const double* __restrict__ acc, float* __res
         out[i] = add(out[i], (float)acc[i]);
 }
 
-// Path-replay adjoint at a Lambert vertex whose albedo is the parameter
-// texture: every contribution after this vertex is linear in its albedo, so
-// d(path radiance)/d(albedo) = (primal radiance - radiance before the vertex)
-// / albedo, per channel; scattered to the four texels of the read.
-__device__ void adjoint_vertex(const PtLaunch& L, const PtSceneTables& T, const PtSurface& sf, uint32_t slot,
-                               uint32_t gprim, float2 mh, float3 alb, const Chan& radBefore)
+// Adjoint at a Lambert vertex whose albedo is the parameter texture: every
+// contribution after this vertex is linear in its albedo, so
+// d(path radiance)/d(albedo) = (path radiance - radiance before the vertex)
+// / albedo, per channel; scattered to the four texels of the read.  A texel's
+// RGBA takes one 16-byte vector reduction (A + 0) where the gradient is
+// 16-byte aligned.
+__device__ __forceinline__ void adjoint_scatter(const PtLaunch& L, const PtSceneTables& T, const PtTexture& tex,
+                                                uint32_t slot, uint32_t gprim, float2 mh, float3 alb, float4 tot,
+                                                float3 before)
 {
-    const float4 tot = L.adj.radTotal[slot];
     const float4 d = L.adj.delta[slot_pixel(L, slot)];
     const float s = L.adj.invSpp;
     const float dd[3] = { d.x, d.y, d.z }, tt[3] = { tot.x, tot.y, tot.z }, aa[3] = { alb.x, alb.y, alb.z };
+    const float rb[3] = { before.x, before.y, before.z };
     float g[3];
 #pragma unroll
     for(int k = 0; k < 3; k++)
-        g[k] = (aa[k] > 0.0f) ? mul(mul(dd[k], s), __fdiv_rn(sub(tt[k], radBefore.v[k]), aa[k])) : 0.0f;
+        g[k] = (aa[k] > 0.0f) ? mul(mul(dd[k], s), __fdiv_rn(sub(tt[k], rb[k]), aa[k])) : 0.0f;
     const float2 uv = surface_uv(T, gprim, mh);
     uint32_t idx[4];
     float w[4];
-    tex_taps(T.textures[sf.tex.x - 1u], uv.x, uv.y, idx, w);
+    tex_taps(tex, uv.x, uv.y, idx, w);
+    const bool vec = (reinterpret_cast<uintptr_t>(L.adj.grad) & 15u) == 0u;
 #pragma unroll
     for(int j = 0; j < 4; j++)
+    {
+        float* q = &L.adj.grad[4 * (size_t)idx[j]];
+        if(vec)
+            atomicAdd(reinterpret_cast<float4*>(q), make_float4(mul(g[0], w[j]), mul(g[1], w[j]), mul(g[2], w[j]), 0.0f));
+        else
 #pragma unroll
-        for(int k = 0; k < 3; k++)
-            atomicAdd(&L.adj.grad[4 * (size_t)idx[j] + k], mul(g[k], w[j]));
+            for(int k = 0; k < 3; k++) atomicAdd(q + k, mul(g[k], w[j]));
+    }
+}
+
+// kAdjRecord: appends the vertex for k_adjoint_scatter, one atomic per group
+// of lanes that got here together.
+__device__ __forceinline__ void adjoint_record(const PtAdjointRecords& R, uint32_t slot, uint32_t gprim, float2 mh,
+                                               float3 alb, const Chan& radBefore)
+{
+    const uint32_t m = __activemask();
+    const uint32_t lane = threadIdx.x & 31u;
+    const int leader = __ffs(m) - 1;
+    uint32_t o = 0;
+    if((int)lane == leader) o = atomicAdd(R.count, (uint32_t)__popc(m));
+    o = __shfl_sync(m, o, leader) + __popc(m & ((1u << lane) - 1u));
+    if(o >= R.cap) return;        // the capacity is slots x maxDepth: not reached
+    R.a[o] = make_float4(__uint_as_float(slot), __uint_as_float(gprim), mh.x, mh.y);
+    R.b[o] = make_float4(alb.x, alb.y, alb.z, radBefore.v[0]);
+    R.c[o] = make_float2(radBefore.v[1], radBefore.v[2]);
 }
 
 // Cache inputs of a surface vertex: position, roughness | outgoing direction |
