@@ -247,7 +247,8 @@ typedef struct mrg_pt_params
                                     group) before every shade, as MRay's
                                     RayPartitioner does: 1 always, 0 never
                                     (shade in hit order), 2 when the scene has
-                                    more than one material group or a skysphere */
+                                    more than one material group or a skysphere
+                                    and a pass has at least 2^18 paths */
     uint32_t sampler;            /* MRG_PT_SAMPLER_*: the paths' random numbers */
     uint32_t samplerMaxSpp;      /* ZSobol initialMaxSampleCount (0: sampleStart + spp) */
 } mrg_pt_params;

@@ -230,26 +230,23 @@ __device__ __noinline__ float mixture_pdf(Mix m, float sumW, float3 d)
 // ---------------------------------------------------------------------------
 template<bool SPEC>
 __global__ void __launch_bounds__(kPtTPB)
-k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T,
-               const uint32_t* __restrict__ aliveList, const uint32_t* __restrict__ aliveCount,
-               uint32_t* nextList, uint32_t* nextCount)
+k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T, PtWork W,
+               uint32_t* nextList, uint32_t* nextCount, uint32_t* shadowCount)
 {
     constexpr int NC = SPEC ? 4 : 3;
     extern __shared__ float gmix[];
     const PtLight* __restrict__ lights = T.lights;
-    const uint32_t n = *aliveCount;
+    const uint32_t n = work_size(W);
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t nAll = L.nLights + (L.env.enabled ? 1u : 0u);
     const float invN = nAll ? __fdiv_rn(1.0f, (float)nAll) : 0.0f;
     const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
     for(uint32_t base = first; base < n; base += stride)
     {
-        const uint32_t idx = base + (threadIdx.x & 31u);
         bool alive = false, shadow = false;
         uint32_t i = 0;
-        if(idx < n)
+        if(work_item(W, base, i))
         {
-            i = aliveList[idx];
             const uint4 hk = P.hits[i];
             const uint32_t st = P.state[i];
             uint32_t depth = st & 0xFFu;
@@ -510,15 +507,15 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
             }
         }
         warp_append(alive, i, nextList, nextCount);
-        warp_append(shadow, i, P.shadowList, P.counts + 2);
+        warp_append(shadow, i, P.shadowList, shadowCount);
     }
 }
 
 // KCAccumulateShadowRaysGPT and KCBackpropagateIrradNEE's records.
 __global__ void __launch_bounds__(kPtTPB)
-k_guide_resolve(PtPaths P, GuidePaths Q)
+k_guide_resolve(PtPaths P, GuidePaths Q, const uint32_t* __restrict__ shadowCount)
 {
-    const uint32_t n = P.counts[2];
+    const uint32_t n = *shadowCount;
     for(uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
     {
         const uint32_t i = P.shadowList[k];
@@ -682,8 +679,8 @@ cudaError_t guide_write_mc(const PtPaths& P, const GuideGrid& G, const GuidePath
 }
 
 cudaError_t guide_shade(const PtLaunch& L, const PtPaths& P, const GuideGrid& G, const GuidePaths& Q,
-                        const PtSceneTables& T, const uint32_t* aliveList, const uint32_t* aliveCount,
-                        uint32_t* nextList, uint32_t* nextCount, int smCount, cudaStream_t st)
+                        const PtSceneTables& T, const PtWork& W, uint32_t* nextList, uint32_t* nextCount,
+                        uint32_t* shadowCount, int smCount, cudaStream_t st)
 {
     static bool attr = false;
     if(!attr)
@@ -698,17 +695,16 @@ cudaError_t guide_shade(const PtLaunch& L, const PtPaths& P, const GuideGrid& G,
     }
     const unsigned grid = (unsigned)smCount * 2u;
     if(L.spec.enabled)
-        k_shade_guided<true><<<grid, kPtTPB, kMixSmem, st>>>(L, P, G, Q, T, aliveList, aliveCount, nextList,
-                                                             nextCount);
+        k_shade_guided<true><<<grid, kPtTPB, kMixSmem, st>>>(L, P, G, Q, T, W, nextList, nextCount, shadowCount);
     else
-        k_shade_guided<false><<<grid, kPtTPB, kMixSmem, st>>>(L, P, G, Q, T, aliveList, aliveCount, nextList,
-                                                              nextCount);
+        k_shade_guided<false><<<grid, kPtTPB, kMixSmem, st>>>(L, P, G, Q, T, W, nextList, nextCount, shadowCount);
     return cudaGetLastError();
 }
 
-cudaError_t guide_resolve(const PtPaths& P, const GuidePaths& Q, int smCount, cudaStream_t st)
+cudaError_t guide_resolve(const PtPaths& P, const GuidePaths& Q, const uint32_t* shadowCount, int smCount,
+                          cudaStream_t st)
 {
-    k_guide_resolve<<<(unsigned)smCount * 4u, kPtTPB, 0, st>>>(P, Q);
+    k_guide_resolve<<<(unsigned)smCount * 4u, kPtTPB, 0, st>>>(P, Q, shadowCount);
     return cudaGetLastError();
 }
 

@@ -91,7 +91,8 @@ struct TraceScene
 
 struct TraceScratch
 {
-    uint32_t*           workCounter = nullptr;   // 1 word, zeroed before each launch
+    uint32_t*           workCounter = nullptr;   // 1 word, zeroed before each launch ...
+    bool                cleared = false;         // ... unless the caller has zeroed it
     uint32_t*           errorFlag = nullptr;     // 1 word, sticky error bits
     unsigned long long* stats = nullptr;         // 8 words (stats kernel only)
 };
@@ -114,6 +115,12 @@ cudaError_t launch_closest(const TraceScene& sc, const TraceScratch& scr, void* 
 cudaError_t launch_visibility(const TraceScene& sc, const TraceScratch& scr, uint32_t* visBits,
                               const void* rays, const uint32_t* rayIdx, uint32_t n,
                               int smCount, cudaStream_t st, const uint32_t* nDevice = nullptr);
+// The shadow rays of a wavefront: any-hit casts of the listed rays; a ray
+// that reaches its light adds its radiance shadowRad[i] to rad[i]
+// (KCAccumulateShadowRaysPT) where the cast ends.
+cudaError_t launch_shadow(const TraceScene& sc, const TraceScratch& scr, const void* rays, const uint32_t* rayIdx,
+                          const uint32_t* nDevice, const float4* shadowRad, float4* rad, int smCount,
+                          cudaStream_t st);
 // Loads the closest-hit traversal kernel on the current device (a function
 // attribute query forces a lazily loaded module in).
 cudaError_t preload_closest();

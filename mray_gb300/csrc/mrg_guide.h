@@ -89,9 +89,10 @@ cudaError_t guide_backprop(const PtLaunch& L, const PtPaths& P, const GuideGrid&
 cudaError_t guide_write_mc(const PtPaths& P, const GuideGrid& G, const GuidePaths& Q, const PtSceneTables& T,
                            const uint32_t* aliveList, const uint32_t* aliveCount, int smCount, cudaStream_t st);
 cudaError_t guide_shade(const PtLaunch& L, const PtPaths& P, const GuideGrid& G, const GuidePaths& Q,
-                        const PtSceneTables& T, const uint32_t* aliveList, const uint32_t* aliveCount,
-                        uint32_t* nextList, uint32_t* nextCount, int smCount, cudaStream_t st);
-cudaError_t guide_resolve(const PtPaths& P, const GuidePaths& Q, int smCount, cudaStream_t st);
+                        const PtSceneTables& T, const PtWork& W, uint32_t* nextList, uint32_t* nextCount,
+                        uint32_t* shadowCount, int smCount, cudaStream_t st);
+cudaError_t guide_resolve(const PtPaths& P, const GuidePaths& Q, const uint32_t* shadowCount, int smCount,
+                          cudaStream_t st);
 // Sorts the bounce's records by (cell, phase) and applies them to the
 // irradiance averages; then marks every record empty for the next bounce.
 cudaError_t guide_apply(const GuideGrid& G, const GuidePaths& Q, int smCount, cudaStream_t st);

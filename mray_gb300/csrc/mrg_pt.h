@@ -184,20 +184,39 @@ struct PtPaths
     uint32_t* listB;
     uint32_t* shadowList;
     uint32_t* shadowLight;   // adjoint: area light of the slot's NEE sample (~0u: the skysphere)
-    uint32_t* counts;        // [0] list A count, [1] list B count, [2] shadow count, [3] pad
-    uint32_t* workKeys;      // work key per alive entry (partitioning)
-    uint32_t* workKeysOut;
-    uint32_t* listSorted;    // alive list grouped by work key
-    uint32_t* sortHist;      // multi-split count table
+    uint32_t* counts;        // kPtCounters words per bounce (PtCounter), zeroed by the pass's raygen
+    uint32_t* groups;        // kPtGroups lists of `capacity`: the alive paths by work group
     uint32_t  capacity;
 };
 
-// Work keys of the partition before shading: miss, light, then one per
+// Work groups of the partition before shading: miss, light, then one per
 // material group (PtMaterial).
-constexpr uint32_t kPtWorkKeyBits = 3;
+constexpr uint32_t kPtGroups = 6;
 
-cudaError_t pt_raygen(const PtLaunch& L, const PtPaths& P, uint32_t* aliveList, uint32_t* aliveCount,
-                      int smCount, cudaStream_t st);
+// Counters of one bounce.  Each bounce has its own, so a pass clears them
+// once instead of a memset before every cast and every shading.
+enum PtCounter : uint32_t
+{
+    kCtrAlive = 0,          // paths that enter the bounce
+    kCtrShadow = 1,         // shadow rays it casts
+    kCtrClaimClosest = 2,   // ray-claim counters of its two casts
+    kCtrClaimShadow = 3,
+    kCtrGroup = 4,          // kPtGroups group sizes
+    kPtCounters = 16
+};
+constexpr uint32_t kPtMaxDepth = 255;
+
+// The paths a shade kernel walks: one list, or the work groups' lists.
+struct PtWork
+{
+    const uint32_t* list;    // nLists lists, `stride` apart
+    const uint32_t* counts;  // their sizes
+    uint32_t        stride;
+    uint32_t        nLists;
+};
+
+// Camera rays of a pass into aliveList; sets the pass's counters.
+cudaError_t pt_raygen(const PtLaunch& L, const PtPaths& P, uint32_t* aliveList, int smCount, cudaStream_t st);
 // Scene tables the shade kernel reads.
 struct PtSceneTables
 {
@@ -210,11 +229,12 @@ struct PtSceneTables
     const PtTexture* textures;
 };
 
-cudaError_t pt_shade_impl(const PtLaunch& L, const PtPaths& P, const PtSceneTables& T,
-                          const uint32_t* aliveList, const uint32_t* aliveCount,
-                          uint32_t* nextList, uint32_t* nextCount, int smCount, cudaStream_t st);
-cudaError_t pt_work_keys(const PtPaths& P, const PtSurface* surfaces, uint32_t nSurfaces,
-                         const uint32_t* aliveList, const uint32_t* aliveCount, int smCount, cudaStream_t st);
+cudaError_t pt_shade_impl(const PtLaunch& L, const PtPaths& P, const PtSceneTables& T, const PtWork& work,
+                          uint32_t* nextList, uint32_t* nextCount, uint32_t* shadowCount, int smCount,
+                          cudaStream_t st);
+// Groups the bounce's alive paths by work group into P.groups / ctr[kCtrGroup..].
+cudaError_t pt_group(const PtLaunch& L, const PtPaths& P, const PtSurface* surfaces, uint32_t nSurfaces,
+                     const uint32_t* aliveList, uint32_t* ctr, cudaStream_t st);
 // rad[slot] += thr[slot] * queryOut[slot] for the queried slots (a
 // spectral path takes the RGB answer at its wavelengths).
 cudaError_t pt_cache_apply(const PtPaths& P, const PtCacheUse& C, const PtSpectral& S, int smCount,
@@ -225,8 +245,10 @@ cudaError_t pt_cache_apply(const PtPaths& P, const PtCacheUse& C, const PtSpectr
 cudaError_t pt_cache_targets(const PtPaths& P, const PtCacheUse& C, const PtSpectral& S, uint32_t slots,
                              float4* batchIn, float4* batchTarget, uint32_t* batchCount, int smCount,
                              cudaStream_t st);
-cudaError_t pt_resolve(const PtLaunch& L, const PtPaths& P, const PtLight* lights, uint32_t depth, int smCount,
-                       cudaStream_t st);
+// Adjoint passes with emission gradients: adds visible NEE samples (P.visBits)
+// to their paths and to the gradient.
+cudaError_t pt_resolve_emission(const PtLaunch& L, const PtPaths& P, const PtLight* lights,
+                                const uint32_t* shadowCount, int smCount, cudaStream_t st);
 // The texture gradient of a pass's vertex records (L.adj.rec), after the pass.
 cudaError_t pt_adjoint_scatter(const PtLaunch& L, const PtPaths& P, const PtSceneTables& T, int smCount,
                                cudaStream_t st);

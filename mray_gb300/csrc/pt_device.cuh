@@ -702,6 +702,30 @@ __device__ __forceinline__ void warp_append(bool pred, uint32_t value, uint32_t*
     if(pred) list[base + __popc(m & ((1u << lane) - 1u))] = value;
 }
 
+// Items of a shade kernel's work: the lists one after another, each padded to
+// whole warps so that no warp holds two groups.
+__device__ __forceinline__ uint32_t work_size(const PtWork& W)
+{
+    if(W.nLists == 1u) return W.counts[0];
+    uint32_t n = 0;
+    for(uint32_t k = 0; k < W.nLists; k++) n += (W.counts[k] + 31u) & ~31u;
+    return n;
+}
+// The path of this lane in the warp at `base` (a multiple of 32), if it has one.
+__device__ __forceinline__ bool work_item(const PtWork& W, uint32_t base, uint32_t& slot)
+{
+    uint32_t k = 0, c = W.counts[0];
+    while(k + 1u < W.nLists && base >= ((c + 31u) & ~31u))
+    {
+        base -= (c + 31u) & ~31u;
+        c = W.counts[++k];
+    }
+    const uint32_t idx = base + (threadIdx.x & 31u);
+    if(idx >= c) return false;
+    slot = W.list[(size_t)k * W.stride + idx];
+    return true;
+}
+
 // throughput * prevPdf / (prevPdf + lightPdf): the balance heuristic with the
 // BxDF pdf cancelled (BalanceCancelled, DistributionFunctions.h:957).
 template<int NC>

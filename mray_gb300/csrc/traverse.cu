@@ -379,7 +379,9 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* __restrict__ 
 // LOCAL: listed ray i starts inside instance instIds[i] (its BLAS, in the
 // instance's space) and ends when that BLAS is exhausted: CastLocalRays.
 // WT: the watertight triangle test on records that hold the three vertices.
-template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false>
+// ADD (with ANY): an unoccluded ray adds its radiance to its path (hits the
+// path radiance, meta the rays' radiance) instead of setting a visibility bit.
+template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false>
 __global__ void __launch_bounds__(kTraceTPB, MRG_TRACE_MIN_BLOCKS)
 k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
         const uint32_t* __restrict__ rayIdx, uint32_t nHost, const uint32_t* __restrict__ nDevice,
@@ -670,6 +672,20 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
                 atomicAdd(&scr.stats[4], (unsigned long long)statTlasNodes);
                 atomicAdd(&scr.stats[5], (unsigned long long)statDry);
             }
+            else if(ADD)
+            {
+                // a separate kernel that read the visibility bits back took
+                // 6 us a bounce at 1M paths, 12 us at 4M, and its launch
+                if(!found)
+                {
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(meta) + ri);
+                    float4* q = reinterpret_cast<float4*>(hits) + ri;
+                    float4 r = *q;
+                    r.x = __fadd_rn(r.x, a.x); r.y = __fadd_rn(r.y, a.y);
+                    r.z = __fadd_rn(r.z, a.z); r.w = __fadd_rn(r.w, a.w);
+                    *q = r;
+                }
+            }
             else if(ANY)
             {
                 const uint32_t bitm = 1u << (ri & 31u);
@@ -689,7 +705,7 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
     }
 }
 
-template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false>
+template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false>
 int blocks_for(int smCount)
 {
     static int perSMOf[kMaxDevices] = {};          // 0: not queried on that device yet
@@ -697,12 +713,17 @@ int blocks_for(int smCount)
     if(perSM == 0)
     {
         int b = 0;
-        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace<ANY, STATS, LOCAL, WT>, kTraceTPB, 0) != cudaSuccess ||
+        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace<ANY, STATS, LOCAL, WT, ADD>, kTraceTPB, 0) != cudaSuccess ||
            b < 1)
             b = 4;
         perSM = b;
     }
     return perSM * smCount;
+}
+
+cudaError_t clear_counter(const TraceScratch& scr, cudaStream_t st)
+{
+    return scr.cleared ? cudaSuccess : cudaMemsetAsync(scr.workCounter, 0, sizeof(uint32_t), st);
 }
 
 } // namespace
@@ -718,7 +739,7 @@ cudaError_t launch_closest(const TraceScene& sc, const TraceScratch& scr, void* 
                            int smCount, cudaStream_t st, const uint32_t* nDevice)
 {
     if(n == 0 && nDevice == nullptr) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(scr.workCounter, 0, sizeof(uint32_t), st);
+    cudaError_t e = clear_counter(scr, st);
     if(e != cudaSuccess) return e;
     if(sc.watertight)
         k_trace<false, false, false, true><<<blocks_for<false, false, false, true>(smCount), kTraceTPB, 0, st>>>(
@@ -753,7 +774,7 @@ cudaError_t launch_visibility(const TraceScene& sc, const TraceScratch& scr, uin
                               int smCount, cudaStream_t st, const uint32_t* nDevice)
 {
     if(n == 0 && nDevice == nullptr) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(scr.workCounter, 0, sizeof(uint32_t), st);
+    cudaError_t e = clear_counter(scr, st);
     if(e != cudaSuccess) return e;
     if(sc.watertight)
         k_trace<true, false, false, true><<<blocks_for<true, false, false, true>(smCount), kTraceTPB, 0, st>>>(
@@ -763,6 +784,24 @@ cudaError_t launch_visibility(const TraceScene& sc, const TraceScratch& scr, uin
         k_trace<true, false><<<blocks_for<true, false>(smCount), kTraceTPB, 0, st>>>(
             sc, scr, const_cast<float4*>(static_cast<const float4*>(rays)), rayIdx, n, nDevice, nullptr,
             nullptr, visBits);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_shadow(const TraceScene& sc, const TraceScratch& scr, const void* rays, const uint32_t* rayIdx,
+                          const uint32_t* nDevice, const float4* shadowRad, float4* rad, int smCount,
+                          cudaStream_t st)
+{
+    cudaError_t e = clear_counter(scr, st);
+    if(e != cudaSuccess) return e;
+    float4* r = const_cast<float4*>(static_cast<const float4*>(rays));
+    uint4* out = reinterpret_cast<uint4*>(rad);
+    float2* add = reinterpret_cast<float2*>(const_cast<float4*>(shadowRad));
+    if(sc.watertight)
+        k_trace<true, false, false, true, true><<<blocks_for<true, false, false, true, true>(smCount), kTraceTPB, 0,
+                                                  st>>>(sc, scr, r, rayIdx, 0, nDevice, out, add, nullptr);
+    else
+        k_trace<true, false, false, false, true><<<blocks_for<true, false, false, false, true>(smCount), kTraceTPB, 0,
+                                                   st>>>(sc, scr, r, rayIdx, 0, nDevice, out, add, nullptr);
     return cudaGetLastError();
 }
 
