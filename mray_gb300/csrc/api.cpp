@@ -80,9 +80,43 @@ void free_accel(mrg_ctx* c)
     cudaFree(c->dTris); c->dTris = nullptr;
     cudaFree(c->dInsts); c->dInsts = nullptr;
     cudaFree(c->dTlasLeaf); c->dTlasLeaf = nullptr;
+    c->capNodes = c->capTris = c->capInsts = c->capTlasLeaf = 0;
     c->blasNodes = c->blasTris = c->tlasNodes = 0;
     c->scene = mrg::TraceScene{};
     c->built = false;
+}
+
+// A result array of at least `bytes`: the one at hand unless it is too small
+// or more than four times too large.
+template<class T>
+cudaError_t ensure(T*& p, size_t& cap, size_t bytes)
+{
+    if(p && cap >= bytes && cap / 4 <= bytes) return cudaSuccess;
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+    if(e == cudaSuccess) cap = bytes;
+    return e;
+}
+
+// Room for `bytes` in the context's mesh blocks (16-byte aligned).
+char* mesh_bytes(mrg_ctx* c, size_t bytes, uint32_t& block)
+{
+    constexpr size_t kBlock = 4u << 20;
+    bytes = (bytes + 15) & ~size_t(15);
+    if(c->meshBlocks.empty() || c->meshBlocks.back().cap - c->meshBlocks.back().used < bytes)
+    {
+        mrg::HostBlock b;
+        b.cap = std::max(bytes, kBlock);
+        b.mem.reset(new char[b.cap]);
+        c->meshBlocks.push_back(std::move(b));
+    }
+    mrg::HostBlock& b = c->meshBlocks.back();
+    block = (uint32_t)(c->meshBlocks.size() - 1);
+    char* p = b.mem.get() + b.used;
+    b.used += bytes;
+    return p;
 }
 
 struct DeviceGuard
@@ -181,6 +215,7 @@ mrg_status mrg_destroy(mrg_ctx* c)
     if(!c) return MRG_OK;
     DeviceGuard g(c->device);
     free_accel(c);
+    c->buildWs.release();
     cudaFree(c->dScratch);
     cudaFree(c->dStats);
     cudaFree(c->dPtSurfaces); cudaFree(c->dPtLights); cudaFree(c->dPtTris); cudaFree(c->ptPathMem);
@@ -224,8 +259,14 @@ mrg_status mrg_upload_mesh(mrg_ctx* c, const float* pos, uint32_t nv, const uint
     mrg_ctx::Mesh m;
     try
     {
-        m.pos.assign(pos, pos + 3ull * nv);
-        m.idx.assign(idx, idx + 3ull * nt);
+        const size_t pb = sizeof(float) * 3ull * nv, ib = sizeof(uint32_t) * 3ull * nt;
+        char* mem = mesh_bytes(c, pb + ib, m.block);
+        m.pos.p = reinterpret_cast<float*>(mem);
+        m.pos.n = 3ull * nv;
+        m.idx.p = reinterpret_cast<uint32_t*>(mem + pb);
+        m.idx.n = 3ull * nt;
+        std::memcpy(m.pos.p, pos, pb);
+        std::memcpy(m.idx.p, idx, ib);
     }
     catch(...) { return fail(MRG_ERR_OUT_OF_MEMORY, "mrg_upload_mesh: host allocation"); }
     m.primKeyBase = primKeyBase;
@@ -270,50 +311,67 @@ mrg_status mrg_build(mrg_ctx* c)
     if(c->insts.empty()) return fail(MRG_ERR_INVALID_ARG, "mrg_build: no instances");
     DeviceGuard g(c->device);
     auto t0 = std::chrono::steady_clock::now();
-    free_accel(c);
+    c->built = false;
+    c->scene = mrg::TraceScene{};
     c->ptDirty = true;
     cudaStream_t st = c->buildStream;
     std::string err;
+    // casts in flight may still read the arrays that the build reuses
+    MRG_TRY(cudaDeviceSynchronize(), "mrg_build: earlier work");
+    mrg::BuildWorkspace& ws = c->buildWs;
+    ws.reset();
+    struct Trim { mrg::BuildWorkspace& w; ~Trim() { w.trim(); } } trim{ ws };
+    auto failed = [&](mrg_status s, const std::string& msg) {
+        cudaStreamSynchronize(st);
+        free_accel(c);
+        return fail(s, msg);
+    };
+    auto cuda_failed = [&](cudaError_t e, const char* what) {
+        cudaStreamSynchronize(st);
+        free_accel(c);
+        return cuda_fail(e, what);
+    };
 
     // 1. BLASes: every mesh in one batched build (PLOC: one build per mesh).
     //    A piece is a node / triangle block placed into the shared arrays;
     //    meshRoot[m] is mesh m's root within its piece.
     struct Piece { mrg::WideNode* nodes; uint32_t nodeCount; mrg::TriRecord* tris; uint32_t payloadCount; };
     std::vector<Piece> pieces;
-    std::vector<uint32_t> pieceOf(c->meshes.size()), meshRoot(c->meshes.size());
-    auto free_pieces = [&]() { for(auto& p : pieces) { cudaFree(p.nodes); cudaFree(p.tris); } };
+    const size_t M = c->meshes.size();
+    std::vector<uint32_t> pieceOf(M), meshRoot(M);
+    uint64_t totalTris = 0;
+    for(const auto& m : c->meshes) totalTris += m.idx.size() / 3;
+    cudaError_t e = ensure(c->dTris, c->capTris, mrg::kTriRecordBytes * totalTris);
+    if(e != cudaSuccess) return cuda_failed(e, "mrg_build: triangle records");
     {
-        const size_t M = c->meshes.size();
-        std::vector<float*> dPos(M, nullptr);
-        std::vector<uint32_t*> dIdx(M, nullptr);
-        auto free_uploads = [&]() { for(size_t i = 0; i < M; i++) { cudaFreeAsync(dPos[i], st); cudaFreeAsync(dIdx[i], st); } };
-        cudaError_t e = cudaSuccess;
-        for(size_t mi = 0; mi < M && e == cudaSuccess; mi++)
+        std::vector<char*> dBlock(c->meshBlocks.size(), nullptr);
+        for(size_t k = 0; k < dBlock.size() && e == cudaSuccess; k++)
         {
-            auto& m = c->meshes[mi];
-            e = cudaMallocAsync(&dPos[mi], sizeof(float) * m.pos.size(), st);
-            if(e == cudaSuccess) e = cudaMallocAsync(&dIdx[mi], sizeof(uint32_t) * m.idx.size(), st);
-            if(e == cudaSuccess) e = cudaMemcpyAsync(dPos[mi], m.pos.data(), sizeof(float) * m.pos.size(), cudaMemcpyHostToDevice, st);
-            if(e == cudaSuccess) e = cudaMemcpyAsync(dIdx[mi], m.idx.data(), sizeof(uint32_t) * m.idx.size(), cudaMemcpyHostToDevice, st);
+            const mrg::HostBlock& b = c->meshBlocks[k];
+            e = ws.take(reinterpret_cast<void**>(&dBlock[k]), b.used);
+            if(e == cudaSuccess) e = cudaMemcpyAsync(dBlock[k], b.mem.get(), b.used, cudaMemcpyHostToDevice, st);
         }
-        if(e != cudaSuccess) { free_uploads(); cudaStreamSynchronize(st); return cuda_fail(e, "mrg_build: mesh upload"); }
+        if(e != cudaSuccess) return cuda_failed(e, "mrg_build: mesh upload");
+        auto on_device = [&](const mrg_ctx::Mesh& m, const void* p) {
+            return dBlock[m.block] + (static_cast<const char*>(p) - c->meshBlocks[m.block].mem.get());
+        };
         if(!use_ploc())
         {
             std::vector<mrg::BatchMeshInput> in(M);
             for(size_t mi = 0; mi < M; mi++)
             {
                 const auto& m = c->meshes[mi];
-                in[mi].pos = dPos[mi]; in[mi].idx = dIdx[mi];
+                in[mi].pos = reinterpret_cast<const float*>(on_device(m, m.pos.p));
+                in[mi].idx = reinterpret_cast<const uint32_t*>(on_device(m, m.idx.p));
                 in[mi].count = (uint32_t)(m.idx.size() / 3);
                 in[mi].primKeyBase = m.primKeyBase;
                 in[mi].maxLeaf = leaf_size(in[mi].count);
                 in[mi].rawVerts = c->watertight;
             }
             mrg::BatchResult br;
-            const bool ok = mrg::build_wide_bvh_batch(in, br, st, err);
-            free_uploads();
-            if(!ok) { cudaStreamSynchronize(st); return fail(MRG_ERR_CUDA, "mrg_build: BLAS build: " + err); }
-            pieces.push_back(Piece{ br.nodes, br.nodeCount, br.tris, br.payloadCount });
+            if(!mrg::build_wide_bvh_batch(in, static_cast<mrg::TriRecord*>(c->dTris), br, ws, st, err))
+                return failed(MRG_ERR_CUDA, "mrg_build: BLAS build: " + err);
+            pieces.push_back(Piece{ br.nodes, br.nodeCount, nullptr, br.payloadCount });
             for(size_t mi = 0; mi < M; mi++)
             {
                 pieceOf[mi] = 0; meshRoot[mi] = (uint32_t)mi;
@@ -326,23 +384,21 @@ mrg_status mrg_build(mrg_ctx* c)
             {
                 auto& m = c->meshes[mi];
                 mrg::BuildInput bi;
-                bi.kind = 0; bi.pos = dPos[mi]; bi.idx = dIdx[mi];
+                bi.kind = 0;
+                bi.pos = reinterpret_cast<const float*>(on_device(m, m.pos.p));
+                bi.idx = reinterpret_cast<const uint32_t*>(on_device(m, m.idx.p));
                 bi.count = (uint32_t)(m.idx.size() / 3);
                 bi.primKeyBase = m.primKeyBase;
                 bi.maxLeaf = leaf_size(bi.count);
                 bi.ploc = true;
                 bi.rawVerts = c->watertight;
                 mrg::BuildResult b;
-                if(!mrg::build_wide_bvh(bi, b, st, err))
-                {
-                    free_uploads(); free_pieces(); cudaStreamSynchronize(st);
-                    return fail(MRG_ERR_CUDA, "mrg_build: BLAS build: " + err);
-                }
+                if(!mrg::build_wide_bvh(bi, b, ws, st, err))
+                    return failed(MRG_ERR_CUDA, "mrg_build: BLAS build: " + err);
                 pieceOf[mi] = (uint32_t)pieces.size(); meshRoot[mi] = 0;
                 pieces.push_back(Piece{ b.nodes, b.nodeCount, b.tris, b.payloadCount });
                 std::memcpy(m.box, b.box, sizeof(m.box));
             }
-            free_uploads();
         }
     }
 
@@ -361,35 +417,23 @@ mrg_status mrg_build(mrg_ctx* c)
     float* dBoxes = nullptr;
     mrg::BuildResult tlas;
     {
-        cudaError_t e = cudaMalloc(&dBoxes, sizeof(float) * instBoxes.size());
+        e = ws.take(reinterpret_cast<void**>(&dBoxes), sizeof(float) * instBoxes.size());
         if(e == cudaSuccess) e = cudaMemcpyAsync(dBoxes, instBoxes.data(), sizeof(float) * instBoxes.size(), cudaMemcpyHostToDevice, st);
-        if(e != cudaSuccess)
-        {
-            cudaFree(dBoxes);
-            free_pieces();
-            return cuda_fail(e, "mrg_build: instance boxes");
-        }
+        if(e != cudaSuccess) return cuda_failed(e, "mrg_build: instance boxes");
         mrg::BuildInput bi;
         bi.kind = 1; bi.boxes = dBoxes; bi.count = ni; bi.maxLeaf = 1;
         bi.ploc = use_ploc();
-        bool ok = mrg::build_wide_bvh(bi, tlas, st, err);
-        cudaFree(dBoxes);
-        if(!ok)
-        {
-            free_pieces();
-            return fail(MRG_ERR_CUDA, "mrg_build: TLAS build: " + err);
-        }
+        if(!mrg::build_wide_bvh(bi, tlas, ws, st, err)) return failed(MRG_ERR_CUDA, "mrg_build: TLAS build: " + err);
     }
 
     // 3. place everything in shared arrays
-    uint64_t totalNodes = 0, totalTris = 0;
-    for(auto& b : pieces) { totalNodes += b.nodeCount; totalTris += b.payloadCount; }
+    uint64_t totalNodes = 0;
+    for(auto& b : pieces) totalNodes += b.nodeCount;
     const uint64_t tlasOff = totalNodes;
     totalNodes += tlas.nodeCount;
-    cudaError_t e = cudaMalloc(&c->dNodes, mrg::kWideNodeBytes * totalNodes);
-    if(e == cudaSuccess) e = cudaMalloc(&c->dTris, mrg::kTriRecordBytes * totalTris);
-    if(e == cudaSuccess) e = cudaMalloc(&c->dInsts, sizeof(mrg::HostInstRecord) * ni);
-    if(e == cudaSuccess) e = cudaMalloc(&c->dTlasLeaf, sizeof(uint32_t) * ni);
+    e = ensure(c->dNodes, c->capNodes, mrg::kWideNodeBytes * totalNodes);
+    if(e == cudaSuccess) e = ensure(c->dInsts, c->capInsts, sizeof(mrg::HostInstRecord) * ni);
+    if(e == cudaSuccess) e = ensure(c->dTlasLeaf, c->capTlasLeaf, sizeof(uint32_t) * ni);
     uint64_t nodeOff = 0, triOff = 0;
     std::vector<uint64_t> pieceNodeOff(pieces.size());
     for(size_t pi = 0; pi < pieces.size() && e == cudaSuccess; pi++)
@@ -400,7 +444,7 @@ mrg_status mrg_build(mrg_ctx* c)
                                     static_cast<char*>(c->dNodes) + mrg::kWideNodeBytes * nodeOff),
                                 b.nodeCount, (uint32_t)nodeOff, (uint32_t)triOff, st))
             e = cudaErrorLaunchFailure;
-        if(e == cudaSuccess)
+        if(e == cudaSuccess && b.tris)
             e = cudaMemcpyAsync(static_cast<char*>(c->dTris) + mrg::kTriRecordBytes * triOff, b.tris,
                                 mrg::kTriRecordBytes * b.payloadCount, cudaMemcpyDeviceToDevice, st);
         nodeOff += b.nodeCount; triOff += b.payloadCount;
@@ -438,9 +482,7 @@ mrg_status mrg_build(mrg_ctx* c)
     if(e == cudaSuccess)
         e = cudaMemcpyAsync(c->dInsts, recs.data(), sizeof(mrg::HostInstRecord) * ni, cudaMemcpyHostToDevice, st);
     if(e == cudaSuccess) e = cudaStreamSynchronize(st);
-    free_pieces();
-    cudaFree(tlas.nodes); cudaFree(tlas.leafIds);
-    if(e != cudaSuccess) { free_accel(c); return cuda_fail(e, "mrg_build: placement"); }
+    if(e != cudaSuccess) return cuda_failed(e, "mrg_build: placement");
 
     c->blasNodes = totalNodes - tlas.nodeCount;
     c->blasTris = totalTris;

@@ -70,6 +70,19 @@ __device__ __forceinline__ uint32_t mesh_of(const uint32_t* __restrict__ firsts,
     return lo;
 }
 
+// What every box of a build is widened by: 1e-5 of the largest coordinate or
+// extent of the root box.
+__host__ __device__ __forceinline__ float box_inflation(const BoxF& b)
+{
+    float ext = 0.0f;
+    for(int k = 0; k < 3; k++)
+    {
+        ext = fmaxf(ext, fmaxf(fabsf(b.mx[k]), fabsf(b.mn[k])));
+        ext = fmaxf(ext, b.mx[k] - b.mn[k]);
+    }
+    return ext * 1.0e-5f + 1.0e-30f;
+}
+
 __device__ __forceinline__ uint32_t f2ord(float f)
 {
     uint32_t u = __float_as_uint(f);
@@ -247,17 +260,23 @@ __global__ void k_morton_multi(const float* __restrict__ cent, const uint32_t* _
     ids[i] = i;
 }
 
-// Root box of every mesh of a batched build (a leaf root for one-triangle meshes).
+// Root box of every mesh of a batched build (a leaf root for one-triangle
+// meshes), its inflation (1e-5 of its extent, as a single build) and its seed
+// in the collapse queue.
 __global__ void k_mesh_boxes(const uint32_t* __restrict__ meshRoot, uint32_t nMesh, const BoxF* __restrict__ nodeBoxes,
                              const BoxF* __restrict__ leafBoxes, const uint32_t* __restrict__ sortedIds, uint32_t n,
-                             BoxF* __restrict__ out, uint32_t* errorFlag)
+                             BoxF* __restrict__ out, MeshSeg* __restrict__ segs, uint4* __restrict__ seeds,
+                             uint32_t* errorFlag)
 {
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if(m >= nMesh) return;
     const uint32_t r = meshRoot[m];
     const uint32_t ix = r & ~kLeafBit;
     if(r == kNoParent || ((r & kLeafBit) ? ix >= n : ix + 1u >= n)) { atomicOr(errorFlag, 1u); return; }
-    out[m] = (r & kLeafBit) ? leafBoxes[sortedIds[ix]] : nodeBoxes[ix];
+    const BoxF b = (r & kLeafBit) ? leafBoxes[sortedIds[ix]] : nodeBoxes[ix];
+    out[m] = b;
+    segs[m].inflate = box_inflation(b);
+    seeds[m] = make_uint4(r, m, m, 0u);
 }
 
 __device__ __forceinline__ int k_delta(const uint64_t* __restrict__ c, int n, int i, int j)
@@ -543,6 +562,12 @@ __global__ void k_ploc_compact(const uint32_t* __restrict__ keep, const uint32_t
     C[o] = inC[i]; CB[o] = inCB[i]; CC[o] = inCC[i];
 }
 
+// Builder counters.  Every level of the collapse has its own queue size, so
+// levels are launched in bursts without asking the host for the next size.
+enum : uint32_t { kCtrNodes = 0, kCtrPayload = 1, kCtrError = 3, kCtrQueue = 4 };
+constexpr uint32_t kMaxLevels = 64;
+constexpr uint32_t kBuildCounters = kCtrQueue + kMaxLevels + 2;
+
 struct CollapseArgs
 {
     const MeshSeg*  segs;       // batched builds: per-mesh payload, leaf size, inflation (else null)
@@ -562,7 +587,7 @@ struct CollapseArgs
     WideNode*       wnodes;
     TriRecord*      tris;
     uint32_t*       leafIds;
-    uint32_t*       counters;   // [0] nodes, [1] leaf payloads, [2] next-queue size, [3] error
+    uint32_t*       counters;   // kCtr*: nodes, leaf payloads, error, then a queue size per level
     uint32_t        leafCount;  // leaves (payload capacity)
     uint32_t        wideCap;    // wide node / queue capacity
     const WideCost* costs;      // SAH-optimal collapse choices (k_wide_cost), or null: greedy
@@ -575,7 +600,7 @@ __device__ __forceinline__ bool ref_ok(const CollapseArgs& a, uint32_t ref)
 {
     const bool ok = (ref & kLeafBit) ? ((ref & ~kLeafBit) < a.leafCount)
                                      : (ref < (a.leafCount > 1 ? a.leafCount - 1 : 1));
-    if(!ok) atomicOr(&a.counters[3], 1u);
+    if(!ok) atomicOr(&a.counters[kCtrError], 1u);
     return ok;
 }
 
@@ -589,7 +614,7 @@ __device__ __forceinline__ void ref_box(const CollapseArgs& a, uint32_t ref, Box
     }
     if(ref & kLeafBit) { b = a.leafBoxes[a.sortedIds[ref & ~kLeafBit]]; cnt = 1; }
     else { b = a.nodeBoxes[ref]; cnt = a.nodes[ref].leafCount; }
-    if(cnt == 0u || cnt > a.leafCount) { atomicOr(&a.counters[3], 1u); cnt = 1; }
+    if(cnt == 0u || cnt > a.leafCount) { atomicOr(&a.counters[kCtrError], 1u); cnt = 1; }
 }
 
 __device__ __forceinline__ float half_area(const BoxF& b)
@@ -632,14 +657,11 @@ __device__ __forceinline__ void emit_payload(const CollapseArgs& a, uint32_t lea
     a.tris[dst] = r;
 }
 
-// One thread per wide node of the current level.  Queue items: binary node
+// One wide node of the current level (k_collapse).  Queue items: binary node
 // (or leaf) reference, wide node index, mesh of a batched build.
-__global__ void k_collapse(CollapseArgs a, const uint4* __restrict__ queue, uint32_t qn,
-                           uint4* __restrict__ nextQueue)
+__device__ __forceinline__ void collapse_node(const CollapseArgs& a, const uint4 item, uint32_t* nextCount,
+                                              uint4* __restrict__ nextQueue)
 {
-    uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if(w >= qn) return;
-    uint4 item = queue[w];
     uint32_t root = item.x;
     uint32_t wideIdx = item.y;
     const uint32_t mesh = item.z;
@@ -691,12 +713,12 @@ __global__ void k_collapse(CollapseArgs a, const uint4* __restrict__ queue, uint
                     continue;
                 }
                 const int k = (int)a.costs[r].split[i - 1];
-                if(k < 1 || k >= i || sp + 2 > 8) { atomicOr(&a.counters[3], 1u); break; }
+                if(k < 1 || k >= i || sp + 2 > 8) { atomicOr(&a.counters[kCtrError], 1u); break; }
                 const BinNode& on = a.nodes[r];
                 stR[sp] = on.right; stI[sp++] = i - k;
                 stR[sp] = on.left;  stI[sp++] = k;
             }
-            if(sp > 0) atomicOr(&a.counters[3], 1u);     // more than 8 children: a malformed table
+            if(sp > 0) atomicOr(&a.counters[kCtrError], 1u);     // more than 8 children: a malformed table
         }
         else
         {
@@ -781,13 +803,13 @@ __global__ void k_collapse(CollapseArgs a, const uint4* __restrict__ queue, uint
         bool leaf = as_leaf(cand[c], ccnt[c]);
         if(leaf) numPayload += ccnt[c]; else numInternal++;
     }
-    uint32_t childBase = numInternal ? atomicAdd(&a.counters[0], numInternal) : 0u;
-    uint32_t triBase = numPayload ? atomicAdd(&a.counters[1], numPayload) : 0u;
-    uint32_t qBase = numInternal ? atomicAdd(&a.counters[2], numInternal) : 0u;
+    uint32_t childBase = numInternal ? atomicAdd(&a.counters[kCtrNodes], numInternal) : 0u;
+    uint32_t triBase = numPayload ? atomicAdd(&a.counters[kCtrPayload], numPayload) : 0u;
+    uint32_t qBase = numInternal ? atomicAdd(nextCount, numInternal) : 0u;
     if(childBase + numInternal > a.wideCap || qBase + numInternal > a.wideCap ||
        triBase + numPayload > a.leafCount || wideIdx >= a.wideCap)
     {
-        atomicOr(&a.counters[3], 2u);
+        atomicOr(&a.counters[kCtrError], 2u);
         return;
     }
 
@@ -835,11 +857,11 @@ __global__ void k_collapse(CollapseArgs a, const uint4* __restrict__ queue, uint
                 if(r & kLeafBit)
                 {
                     if(m < k) emit_payload(a, r & ~kLeafBit, triBase + triOff + m, mesh);
-                    else atomicOr(&a.counters[3], 4u);
+                    else atomicOr(&a.counters[kCtrError], 4u);
                     m++;
                 }
                 else if(sp + 2 <= 8) { stack[sp++] = a.nodes[r].right; stack[sp++] = a.nodes[r].left; }
-                else atomicOr(&a.counters[3], 4u);
+                else atomicOr(&a.counters[kCtrError], 4u);
             }
             triOff += k;
         }
@@ -859,6 +881,15 @@ __global__ void k_collapse(CollapseArgs a, const uint4* __restrict__ queue, uint
         out.q[k] = make_uint4(pair(0), pair(2), pair(4), pair(6));
     }
     a.wnodes[wideIdx] = out;
+}
+
+// One thread per wide node of a level.
+__global__ void k_collapse(CollapseArgs a, uint32_t level, const uint4* __restrict__ queue,
+                           uint4* __restrict__ nextQueue)
+{
+    const uint32_t qn = min(a.counters[kCtrQueue + level], a.wideCap);
+    for(uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < qn; w += gridDim.x * blockDim.x)
+        collapse_node(a, queue[w], &a.counters[kCtrQueue + level + 1u], nextQueue);
 }
 
 // Adds fixed offsets to child / payload bases when a build is placed into the
@@ -920,7 +951,106 @@ float sah_cprim() { return env_cost("MRG_BVH_SAH_CPRIM", 1.0f); }
 float sah_cinst() { return env_cost("MRG_BVH_SAH_CINST", 8.0f); }
 } // namespace
 
-bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std::string& err)
+void BuildWorkspace::reset() { for(Slab& s : slabs_) s.used = 0; }
+
+cudaError_t BuildWorkspace::take(void** out, size_t bytes)
+{
+    bytes = (std::max<size_t>(bytes, 1) + 255) & ~size_t(255);
+    for(Slab& s : slabs_)
+        if(s.cap - s.used >= bytes)
+        {
+            *out = s.mem + s.used;
+            s.used += bytes;
+            return cudaSuccess;
+        }
+    const size_t cap = std::max(bytes, size_t(4) << 20);
+    char* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, cap);
+    if(e != cudaSuccess) return e;
+    slabs_.push_back(Slab{ mem, cap, bytes });
+    *out = mem;
+    return cudaSuccess;
+}
+
+void BuildWorkspace::trim()
+{
+    size_t total = 0;
+    for(const Slab& s : slabs_) total += s.cap;
+    if(total > kKeepBytes) release();
+}
+
+void BuildWorkspace::release()
+{
+    for(Slab& s : slabs_) cudaFree(s.mem);
+    slabs_.clear();
+}
+
+namespace {
+
+// The arrays of one build, one piece of the workspace.
+class Carve
+{
+public:
+    template<class T>
+    void add(T*& p, size_t n)
+    {
+        items_.push_back({ reinterpret_cast<void**>(&p), bytes_ });
+        bytes_ += (sizeof(T) * std::max<size_t>(n, 1) + 255) & ~size_t(255);
+    }
+    cudaError_t take(BuildWorkspace& ws)
+    {
+        void* base = nullptr;
+        cudaError_t e = ws.take(&base, bytes_);
+        if(e != cudaSuccess) return e;
+        for(const Item& i : items_) *i.p = static_cast<char*>(base) + i.off;
+        return cudaSuccess;
+    }
+private:
+    struct Item { void** p; size_t off; };
+    std::vector<Item> items_;
+    size_t bytes_ = 0;
+};
+
+// Collapse, level by level from the seeds already in q[0] (their number in
+// counters[kCtrQueue]).  Levels go out in bursts; a level past the last finds
+// an empty queue (2 us), where a read-back per level cost 20 us.
+bool collapse(const CollapseArgs& ca, uint4* const q[2], cudaStream_t st, uint32_t (&host)[kBuildCounters],
+              std::string& err)
+{
+    const unsigned grid = std::min(gridFor(ca.wideCap, 128), 152u * 16u);
+    for(uint32_t level = 0;;)
+    {
+        const uint32_t end = std::min(level + (level ? 4u : 8u), kMaxLevels + 1u);
+        for(; level < end; level++) k_collapse<<<grid, 128, 0, st>>>(ca, level, q[level & 1u], q[(level & 1u) ^ 1u]);
+        MRG_CK(cudaGetLastError());
+        MRG_CK(cudaMemcpyAsync(host, ca.counters, sizeof(host), cudaMemcpyDeviceToHost, st));
+        MRG_CK(cudaStreamSynchronize(st));
+        if(host[kCtrError] != 0) { err = "wide BVH collapse reported an invalid tree"; goto fail; }
+        if(host[kCtrNodes] > ca.wideCap) { err = "wide node capacity exceeded"; goto fail; }
+        if(host[kCtrQueue + level] == 0) break;
+        if(level > kMaxLevels) { err = "wide BVH deeper than 64 levels"; goto fail; }
+    }
+    if(host[kCtrPayload] != ca.leafCount) { err = "payload count mismatch"; goto fail; }
+    return true;
+fail:
+    return false;
+}
+
+// Radix sort of (code, leaf) by the low `endBit` bits; scratch from the workspace.
+cudaError_t sort_codes(cub::DoubleBuffer<uint64_t>& kb, cub::DoubleBuffer<uint32_t>& vb, uint32_t n, int endBit,
+                       BuildWorkspace& ws, cudaStream_t st)
+{
+    size_t bytes = 0;
+    void* temp = nullptr;
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, (int)n, 0, endBit, st);
+    if(e == cudaSuccess) e = ws.take(&temp, bytes);
+    if(e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(temp, bytes, kb, vb, (int)n, 0, endBit, st);
+    return e;
+}
+
+} // namespace
+
+bool build_wide_bvh(const BuildInput& in, BuildResult& out, BuildWorkspace& ws, cudaStream_t st, std::string& err)
 {
     const uint32_t n = in.count;
     out = BuildResult{};
@@ -928,7 +1058,6 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
 
     BoxF* dLeafBoxes = nullptr; float* dCent = nullptr; uint32_t* dCB = nullptr;
     uint64_t* dCodes[2] = { nullptr, nullptr }; uint32_t* dIds[2] = { nullptr, nullptr };
-    void* dTemp = nullptr; size_t tempBytes = 0;
     BinNode* dNodes = nullptr; BoxF* dNodeBoxes = nullptr; uint32_t* dLeafParent = nullptr; WideCost* dCosts = nullptr;
     uint32_t* dCnt = nullptr; uint4* dQ[2] = { nullptr, nullptr };
     uint32_t* dCounters = nullptr;
@@ -936,35 +1065,26 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
     const uint32_t nInt = (n > 1) ? (n - 1) : 1;
     const uint32_t wideCap = n;      // each wide node consumes >= 1 binary node
     uint32_t cbInit[6] = { 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u };
-    uint32_t hostCounters[4];
+    uint32_t hostCounters[kBuildCounters] = {};
     BoxF rootBox;
     cub::DoubleBuffer<uint64_t> kb;
     cub::DoubleBuffer<uint32_t> vb;
-    uint32_t qn = 1;
-    int cur = 0;
     uint4 rootItem;
     CollapseArgs ca;
-    float ext;
+    Carve carve;
+    const bool sah = n > 1 && !in.ploc && in.maxLeaf <= sah_max_leaf(in.kind == 1);
 
-    MRG_CK(cudaMallocAsync(&dLeafBoxes, sizeof(BoxF) * n, st));
-    MRG_CK(cudaMallocAsync(&dCent, sizeof(float) * 3 * n, st));
-    MRG_CK(cudaMallocAsync(&dCB, sizeof(uint32_t) * 6, st));
-    MRG_CK(cudaMallocAsync(&dCodes[0], sizeof(uint64_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dCodes[1], sizeof(uint64_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dIds[0], sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dIds[1], sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dNodes, sizeof(BinNode) * nInt, st));
-    MRG_CK(cudaMallocAsync(&dNodeBoxes, sizeof(BoxF) * nInt, st));
-    MRG_CK(cudaMallocAsync(&dLeafParent, sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dCnt, sizeof(uint32_t) * nInt, st));
-    MRG_CK(cudaMallocAsync(&dQ[0], sizeof(uint4) * wideCap, st));
-    MRG_CK(cudaMallocAsync(&dQ[1], sizeof(uint4) * wideCap, st));
-    MRG_CK(cudaMallocAsync(&dCounters, sizeof(uint32_t) * 4, st));
-    MRG_CK(cudaMallocAsync(&dW, sizeof(WideNode) * wideCap, st));
-    if(in.kind == 0) MRG_CK(cudaMallocAsync(&out.tris, sizeof(TriRecord) * n, st));
-    else             MRG_CK(cudaMallocAsync(&out.leafIds, sizeof(uint32_t) * n, st));
+    carve.add(dLeafBoxes, n); carve.add(dCent, 3ull * n); carve.add(dCB, 6);
+    carve.add(dCodes[0], n); carve.add(dCodes[1], n); carve.add(dIds[0], n); carve.add(dIds[1], n);
+    carve.add(dNodes, nInt); carve.add(dNodeBoxes, nInt); carve.add(dLeafParent, n); carve.add(dCnt, nInt);
+    carve.add(dQ[0], wideCap); carve.add(dQ[1], wideCap); carve.add(dCounters, kBuildCounters);
+    carve.add(dW, wideCap);
+    if(sah) carve.add(dCosts, nInt);
+    if(in.kind == 0) carve.add(out.tris, n); else carve.add(out.leafIds, n);
+    MRG_CK(carve.take(ws));
 
     MRG_CK(cudaMemcpyAsync(dCB, cbInit, sizeof(cbInit), cudaMemcpyHostToDevice, st));
+    MRG_CK(cudaMemsetAsync(dCounters, 0, sizeof(uint32_t) * kBuildCounters, st));
     if(in.kind == 0)
         k_leaf_boxes_tri<<<gridFor(n), kTPB, 0, st>>>(in.pos, in.idx, n, dLeafBoxes, dCent, dCB);
     else
@@ -976,9 +1096,7 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
 
     kb = cub::DoubleBuffer<uint64_t>(dCodes[0], dCodes[1]);
     vb = cub::DoubleBuffer<uint32_t>(dIds[0], dIds[1]);
-    MRG_CK(cub::DeviceRadixSort::SortPairs(nullptr, tempBytes, kb, vb, (int)n, 0, 63, st));
-    MRG_CK(cudaMallocAsync(&dTemp, tempBytes, st));
-    MRG_CK(cub::DeviceRadixSort::SortPairs(dTemp, tempBytes, kb, vb, (int)n, 0, 63, st));
+    MRG_CK(sort_codes(kb, vb, n, 63, ws, st));
 
     if(n > 1 && in.ploc)
     {
@@ -1000,7 +1118,7 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
               cudaMallocAsync(&dPos, sizeof(uint32_t) * n, st) == cudaSuccess &&
               cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, dKeep, dPos, (int)n, st) == cudaSuccess &&
               cudaMallocAsync(&dScanTemp, scanBytes, st) == cudaSuccess;
-        okP = okP && cudaMemsetAsync(dCounters, 0, sizeof(uint32_t) * 4, st) == cudaSuccess;
+        okP = okP && cudaMemsetAsync(dCounters, 0, sizeof(uint32_t) * kBuildCounters, st) == cudaSuccess;
         if(okP) k_ploc_init<<<gridFor(n), kTPB, 0, st>>>(vb.Current(), dLeafBoxes, n, dC[0], dCB[0], dCC[0]);
         uint32_t cn = n;
         int pc = 0;
@@ -1010,7 +1128,7 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
             k_ploc_nearest<<<gridFor(cn), kTPB, 0, st>>>(dCB[pc], cn, dNN);
             k_ploc_merge<<<gridFor(cn), kTPB, 0, st>>>(dC[pc], dCB[pc], dCC[pc], dNN, cn, dNodes, dNodeBoxes,
                                                        dCounters + 0, nInt, dC[pc ^ 1], dCB[pc ^ 1], dCC[pc ^ 1],
-                                                       dKeep, dCounters + 3);
+                                                       dKeep, dCounters + kCtrError);
             okP = cub::DeviceScan::ExclusiveSum(dScanTemp, scanBytes, dKeep, dPos, (int)cn, st) == cudaSuccess;
             uint32_t lastKeep = 0, lastPos = 0;
             okP = okP && cudaMemcpyAsync(&lastKeep, dKeep + cn - 1, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
@@ -1038,17 +1156,15 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
         k_karras<<<gridFor(n - 1), kTPB, 0, st>>>(kb.Current(), (int)n, dNodes, dLeafParent, nullptr, 0u, nullptr);
         MRG_CK(cudaGetLastError());
         MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
-        MRG_CK(cudaMemsetAsync(dCounters, 0, sizeof(uint32_t) * 4, st));
         k_bottom_up<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes,
-                                                 dNodeBoxes, dCnt, (int)n, dCounters + 3);
+                                                 dNodeBoxes, dCnt, (int)n, dCounters + kCtrError);
         MRG_CK(cudaGetLastError());
-        if(in.maxLeaf <= sah_max_leaf(in.kind == 1))
+        if(sah)
         {
-            MRG_CK(cudaMallocAsync(&dCosts, sizeof(WideCost) * nInt, st));
             MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
             k_wide_cost<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes, dNodeBoxes,
                                                      dCosts, dCnt, (int)n, nullptr, nullptr, 0u, in.maxLeaf, 1.0f,
-                                                     in.kind == 1 ? sah_cinst() : sah_cprim(), dCounters + 3);
+                                                     in.kind == 1 ? sah_cinst() : sah_cprim(), dCounters + kCtrError);
             MRG_CK(cudaGetLastError());
         }
         MRG_CK(cudaMemcpyAsync(&rootBox, dNodeBoxes, sizeof(BoxF), cudaMemcpyDeviceToHost, st));
@@ -1059,91 +1175,51 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std
         MRG_CK(cudaMemcpyAsync(&rootBox, dLeafBoxes, sizeof(BoxF), cudaMemcpyDeviceToHost, st));
         rootItem = make_uint4(kLeafBit | 0u, 0u, 0u, 0u);
     }
-    MRG_CK(cudaMemcpyAsync(hostCounters, dCounters, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st));
+    MRG_CK(cudaMemcpyAsync(hostCounters, dCounters, sizeof(hostCounters), cudaMemcpyDeviceToHost, st));
     MRG_CK(cudaStreamSynchronize(st));
-    if(n > 1 && hostCounters[3] != 0) { err = "binary tree construction produced an invalid node"; goto fail; }
+    if(hostCounters[kCtrError] != 0) { err = "binary tree construction produced an invalid node"; goto fail; }
     for(int k = 0; k < 3; k++) { out.box[k] = rootBox.mn[k]; out.box[3 + k] = rootBox.mx[k]; }
-
-    ext = 0.0f;
-    for(int k = 0; k < 3; k++)
-    {
-        float e = fabsf(rootBox.mx[k]) > fabsf(rootBox.mn[k]) ? fabsf(rootBox.mx[k]) : fabsf(rootBox.mn[k]);
-        ext = (ext > e) ? ext : e;
-        float sp = rootBox.mx[k] - rootBox.mn[k];
-        ext = (ext > sp) ? ext : sp;
-    }
 
     ca.segs = nullptr;
     ca.nodes = dNodes; ca.nodeBoxes = dNodeBoxes; ca.leafBoxes = dLeafBoxes;
     ca.sortedIds = vb.Current(); ca.pos = in.pos; ca.idx = in.idx;
     ca.primKeyBase = in.primKeyBase; ca.kind = in.kind; ca.maxLeaf = in.maxLeaf;
     ca.rawVerts = in.rawVerts ? 1u : 0u;
-    ca.inflate = ext * 1.0e-5f + 1.0e-30f;
+    ca.inflate = box_inflation(rootBox);
     ca.wnodes = dW; ca.tris = out.tris; ca.leafIds = out.leafIds; ca.counters = dCounters;
     ca.leafCount = n; ca.wideCap = wideCap;
     ca.costs = dCosts; ca.sahMaxLeaf = dCosts ? 3u : 0u;
 
-    hostCounters[0] = 1; hostCounters[1] = 0; hostCounters[2] = 0; hostCounters[3] = 0;
+    std::fill(hostCounters, hostCounters + kBuildCounters, 0u);
+    hostCounters[kCtrNodes] = 1;
+    hostCounters[kCtrQueue] = 1;
     MRG_CK(cudaMemcpyAsync(dCounters, hostCounters, sizeof(hostCounters), cudaMemcpyHostToDevice, st));
     MRG_CK(cudaMemcpyAsync(dQ[0], &rootItem, sizeof(uint4), cudaMemcpyHostToDevice, st));
-    for(int level = 0; qn > 0; level++)
-    {
-        if(level > 64) { err = "wide BVH deeper than 64 levels"; goto fail; }
-        MRG_CK(cudaMemsetAsync(dCounters + 2, 0, sizeof(uint32_t), st));
-        k_collapse<<<gridFor(qn, 128), 128, 0, st>>>(ca, dQ[cur], qn, dQ[cur ^ 1]);
-        MRG_CK(cudaGetLastError());
-        MRG_CK(cudaMemcpyAsync(hostCounters, dCounters, sizeof(hostCounters), cudaMemcpyDeviceToHost, st));
-        MRG_CK(cudaStreamSynchronize(st));
-        if(hostCounters[3] != 0) { err = "wide BVH collapse reported an invalid tree"; goto fail; }
-        if(hostCounters[0] > wideCap) { err = "wide node capacity exceeded"; goto fail; }
-        qn = hostCounters[2];
-        cur ^= 1;
-    }
-    if(hostCounters[1] != n) { err = "payload count mismatch"; goto fail; }
-    out.nodeCount = hostCounters[0];
-    MRG_CK(cudaMallocAsync(&out.nodes, sizeof(WideNode) * out.nodeCount, st));
-    MRG_CK(cudaMemcpyAsync(out.nodes, dW, sizeof(WideNode) * out.nodeCount, cudaMemcpyDeviceToDevice, st));
+    if(!collapse(ca, dQ, st, hostCounters, err)) goto fail;
+    out.nodes = dW;
+    out.nodeCount = hostCounters[kCtrNodes];
     out.payloadCount = n;
-
-    cudaFreeAsync(dLeafBoxes, st); cudaFreeAsync(dCent, st); cudaFreeAsync(dCB, st);
-    cudaFreeAsync(dCodes[0], st); cudaFreeAsync(dCodes[1], st);
-    cudaFreeAsync(dIds[0], st); cudaFreeAsync(dIds[1], st); cudaFreeAsync(dTemp, st);
-    cudaFreeAsync(dNodes, st); cudaFreeAsync(dNodeBoxes, st); cudaFreeAsync(dLeafParent, st);
-    cudaFreeAsync(dCnt, st); cudaFreeAsync(dQ[0], st); cudaFreeAsync(dQ[1], st);
-    cudaFreeAsync(dCounters, st); cudaFreeAsync(dW, st); cudaFreeAsync(dCosts, st);
-    if(cudaStreamSynchronize(st) != cudaSuccess) { err = "stream sync failed"; return false; }
     return true;
 
 fail:
     cudaStreamSynchronize(st);
-    cudaFree(dLeafBoxes); cudaFree(dCent); cudaFree(dCB); cudaFree(dCodes[0]); cudaFree(dCodes[1]);
-    cudaFree(dIds[0]); cudaFree(dIds[1]); cudaFree(dTemp); cudaFree(dNodes); cudaFree(dNodeBoxes);
-    cudaFree(dLeafParent); cudaFree(dCnt); cudaFree(dQ[0]); cudaFree(dQ[1]); cudaFree(dCounters);
-    cudaFree(dW); cudaFree(dCosts); cudaFree(out.nodes); cudaFree(out.tris); cudaFree(out.leafIds);
     out = BuildResult{};
     return false;
 }
 
-bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, BatchResult& out, cudaStream_t st,
-                          std::string& err)
+bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, TriRecord* tris, BatchResult& out,
+                          BuildWorkspace& ws, cudaStream_t st, std::string& err)
 {
     out = BatchResult{};
     const uint32_t M = (uint32_t)meshes.size();
     if(M == 0) { err = "empty batch"; return false; }
-    std::vector<uint32_t> firsts(M + 1);
-    std::vector<MeshSeg> segs(M);
     uint64_t total = 0;
-    for(uint32_t m = 0; m < M; m++)
+    for(const BatchMeshInput& in : meshes)
     {
-        const BatchMeshInput& in = meshes[m];
         if(in.count == 0 || !in.pos || !in.idx) { err = "empty mesh in batch"; return false; }
-        firsts[m] = (uint32_t)total;
-        segs[m] = MeshSeg{ in.pos, in.idx, (uint32_t)total, in.count, in.primKeyBase,
-                           std::min(3u, std::max(1u, in.maxLeaf)), 0.0f, in.rawVerts ? 1u : 0u };
         total += in.count;
         if(total >= (1ull << 31)) { err = "batch larger than 2^31 triangles"; return false; }
     }
-    firsts[M] = (uint32_t)total;
     const uint32_t n = (uint32_t)total;
     const uint32_t nInt = (n > 1) ? (n - 1) : 1;
     const uint32_t wideCap = n;
@@ -1153,65 +1229,68 @@ bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, BatchResult
     const uint32_t bits = std::min(21u, (64u - mbits) / 3u);
     const int endBit = (int)(mbits + 3u * bits);
 
-    MeshSeg* dSegs = nullptr; uint32_t* dFirsts = nullptr; uint32_t* dCB = nullptr; uint32_t* dLeafMesh = nullptr;
+    // per-mesh tables, one upload: segments, first leaves, centroid bounds, roots
+    const size_t segBytes = (sizeof(MeshSeg) * M + 15) & ~size_t(15);
+    const size_t tableBytes = segBytes + sizeof(uint32_t) * ((size_t)M + 1 + 6ull * M + M);
+    std::vector<char> table(tableBytes);
+    MeshSeg* segs = reinterpret_cast<MeshSeg*>(table.data());
+    uint32_t* firsts = reinterpret_cast<uint32_t*>(table.data() + segBytes);
+    uint32_t* cbInit = firsts + M + 1;
+    uint32_t* meshRoot = cbInit + 6ull * M;
+    uint32_t first = 0;
+    for(uint32_t m = 0; m < M; m++)
+    {
+        const BatchMeshInput& in = meshes[m];
+        firsts[m] = first;
+        segs[m] = MeshSeg{ in.pos, in.idx, first, in.count, in.primKeyBase,
+                           std::min(3u, std::max(1u, in.maxLeaf)), 0.0f, in.rawVerts ? 1u : 0u };
+        for(int k = 0; k < 3; k++) { cbInit[6 * m + k] = 0xFFFFFFFFu; cbInit[6 * m + 3 + k] = 0u; }
+        meshRoot[m] = (in.count == 1u) ? (kLeafBit | first) : kNoParent;
+        first += in.count;
+    }
+    firsts[M] = n;
+
+    char* dTable = nullptr; uint32_t* dLeafMesh = nullptr;
     BoxF* dLeafBoxes = nullptr; float* dCent = nullptr;
     uint64_t* dCodes[2] = { nullptr, nullptr }; uint32_t* dIds[2] = { nullptr, nullptr };
-    void* dTemp = nullptr; size_t tempBytes = 0;
     BinNode* dNodes = nullptr; BoxF* dNodeBoxes = nullptr; uint32_t* dLeafParent = nullptr; WideCost* dCosts = nullptr;
     uint32_t* dCnt = nullptr; uint4* dQ[2] = { nullptr, nullptr };
-    uint32_t* dCounters = nullptr; uint32_t* dMeshRoot = nullptr; BoxF* dMeshBoxes = nullptr;
+    uint32_t* dCounters = nullptr; BoxF* dMeshBoxes = nullptr;
     WideNode* dW = nullptr;
-    std::vector<uint32_t> cbInit(6ull * M), meshRoot(M);
+    MeshSeg* dSegs = nullptr;
+    uint32_t *dFirsts = nullptr, *dCB = nullptr, *dMeshRoot = nullptr;
     std::vector<BoxF> meshBoxes(M);
-    std::vector<uint4> seeds(M);
-    uint32_t hostCounters[4] = { 0, 0, 0, 0 };
+    uint32_t hostCounters[kBuildCounters] = {};
     cub::DoubleBuffer<uint64_t> kb;
     cub::DoubleBuffer<uint32_t> vb;
     CollapseArgs ca;
-    uint32_t qn = M;
-    int cur = 0;
+    Carve carve;
+    const bool sah = n > 1 && sah_max_leaf(false) > 0u;
 
-    for(uint32_t m = 0; m < M; m++)
-    {
-        for(int k = 0; k < 3; k++) { cbInit[6 * m + k] = 0xFFFFFFFFu; cbInit[6 * m + 3 + k] = 0u; }
-        meshRoot[m] = (segs[m].count == 1u) ? (kLeafBit | segs[m].first) : kNoParent;
-    }
-    MRG_CK(cudaMallocAsync(&dSegs, sizeof(MeshSeg) * M, st));
-    MRG_CK(cudaMallocAsync(&dFirsts, sizeof(uint32_t) * (M + 1), st));
-    MRG_CK(cudaMallocAsync(&dCB, sizeof(uint32_t) * 6 * M, st));
-    MRG_CK(cudaMallocAsync(&dLeafMesh, sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dLeafBoxes, sizeof(BoxF) * n, st));
-    MRG_CK(cudaMallocAsync(&dCent, sizeof(float) * 3 * n, st));
-    MRG_CK(cudaMallocAsync(&dCodes[0], sizeof(uint64_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dCodes[1], sizeof(uint64_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dIds[0], sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dIds[1], sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dNodes, sizeof(BinNode) * nInt, st));
-    MRG_CK(cudaMallocAsync(&dNodeBoxes, sizeof(BoxF) * nInt, st));
-    MRG_CK(cudaMallocAsync(&dLeafParent, sizeof(uint32_t) * n, st));
-    MRG_CK(cudaMallocAsync(&dCnt, sizeof(uint32_t) * nInt, st));
-    MRG_CK(cudaMallocAsync(&dQ[0], sizeof(uint4) * wideCap, st));
-    MRG_CK(cudaMallocAsync(&dQ[1], sizeof(uint4) * wideCap, st));
-    MRG_CK(cudaMallocAsync(&dCounters, sizeof(uint32_t) * 4, st));
-    MRG_CK(cudaMallocAsync(&dMeshRoot, sizeof(uint32_t) * M, st));
-    MRG_CK(cudaMallocAsync(&dMeshBoxes, sizeof(BoxF) * M, st));
-    MRG_CK(cudaMallocAsync(&dW, sizeof(WideNode) * wideCap, st));
-    MRG_CK(cudaMallocAsync(&out.tris, sizeof(TriRecord) * n, st));
+    carve.add(dTable, tableBytes); carve.add(dLeafMesh, n);
+    carve.add(dLeafBoxes, n); carve.add(dCent, 3ull * n);
+    carve.add(dCodes[0], n); carve.add(dCodes[1], n); carve.add(dIds[0], n); carve.add(dIds[1], n);
+    carve.add(dNodes, nInt); carve.add(dNodeBoxes, nInt); carve.add(dLeafParent, n); carve.add(dCnt, nInt);
+    carve.add(dQ[0], wideCap); carve.add(dQ[1], wideCap); carve.add(dCounters, kBuildCounters);
+    carve.add(dMeshBoxes, M); carve.add(dW, wideCap);
+    if(sah) carve.add(dCosts, nInt);
+    MRG_CK(carve.take(ws));
+    dSegs = reinterpret_cast<MeshSeg*>(dTable);
+    dFirsts = reinterpret_cast<uint32_t*>(dTable + segBytes);
+    dCB = dFirsts + M + 1;
+    dMeshRoot = dCB + 6ull * M;
 
-    MRG_CK(cudaMemcpyAsync(dSegs, segs.data(), sizeof(MeshSeg) * M, cudaMemcpyHostToDevice, st));
-    MRG_CK(cudaMemcpyAsync(dFirsts, firsts.data(), sizeof(uint32_t) * (M + 1), cudaMemcpyHostToDevice, st));
-    MRG_CK(cudaMemcpyAsync(dCB, cbInit.data(), sizeof(uint32_t) * 6 * M, cudaMemcpyHostToDevice, st));
-    MRG_CK(cudaMemcpyAsync(dMeshRoot, meshRoot.data(), sizeof(uint32_t) * M, cudaMemcpyHostToDevice, st));
-    MRG_CK(cudaMemsetAsync(dCounters, 0, sizeof(uint32_t) * 4, st));
+    hostCounters[kCtrNodes] = M;
+    hostCounters[kCtrQueue] = M;
+    MRG_CK(cudaMemcpyAsync(dTable, table.data(), tableBytes, cudaMemcpyHostToDevice, st));
+    MRG_CK(cudaMemcpyAsync(dCounters, hostCounters, sizeof(hostCounters), cudaMemcpyHostToDevice, st));
     k_leaf_boxes_multi<<<gridFor(n), kTPB, 0, st>>>(dSegs, dFirsts, M, n, dLeafBoxes, dCent, dCB, dLeafMesh);
     MRG_CK(cudaGetLastError());
     k_morton_multi<<<gridFor(n), kTPB, 0, st>>>(dCent, dCB, dLeafMesh, n, bits, dCodes[0], dIds[0]);
     MRG_CK(cudaGetLastError());
     kb = cub::DoubleBuffer<uint64_t>(dCodes[0], dCodes[1]);
     vb = cub::DoubleBuffer<uint32_t>(dIds[0], dIds[1]);
-    MRG_CK(cub::DeviceRadixSort::SortPairs(nullptr, tempBytes, kb, vb, (int)n, 0, endBit, st));
-    MRG_CK(cudaMallocAsync(&dTemp, tempBytes, st));
-    MRG_CK(cub::DeviceRadixSort::SortPairs(dTemp, tempBytes, kb, vb, (int)n, 0, endBit, st));
+    MRG_CK(sort_codes(kb, vb, n, endBit, ws, st));
     if(n > 1)
     {
         MRG_CK(cudaMemsetAsync(dNodes, 0xFF, sizeof(BinNode) * nInt, st));
@@ -1220,94 +1299,47 @@ bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, BatchResult
         MRG_CK(cudaGetLastError());
         MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
         k_bottom_up<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes,
-                                                 dNodeBoxes, dCnt, (int)n, dCounters + 3);
+                                                 dNodeBoxes, dCnt, (int)n, dCounters + kCtrError);
         MRG_CK(cudaGetLastError());
-        if(sah_max_leaf(false) > 0u)
+        if(sah)
         {
-            MRG_CK(cudaMallocAsync(&dCosts, sizeof(WideCost) * nInt, st));
             MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
             k_wide_cost<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes, dNodeBoxes,
                                                      dCosts, dCnt, (int)n, dFirsts, dSegs, M, 3u, 1.0f,
-                                                     sah_cprim(), dCounters + 3);
+                                                     sah_cprim(), dCounters + kCtrError);
             MRG_CK(cudaGetLastError());
         }
     }
     k_mesh_boxes<<<gridFor(M), kTPB, 0, st>>>(dMeshRoot, M, dNodeBoxes, dLeafBoxes, vb.Current(), n, dMeshBoxes,
-                                              dCounters + 3);
+                                              dSegs, dQ[0], dCounters + kCtrError);
     MRG_CK(cudaGetLastError());
-    MRG_CK(cudaMemcpyAsync(meshRoot.data(), dMeshRoot, sizeof(uint32_t) * M, cudaMemcpyDeviceToHost, st));
     MRG_CK(cudaMemcpyAsync(meshBoxes.data(), dMeshBoxes, sizeof(BoxF) * M, cudaMemcpyDeviceToHost, st));
     MRG_CK(cudaMemcpyAsync(hostCounters, dCounters, sizeof(hostCounters), cudaMemcpyDeviceToHost, st));
     MRG_CK(cudaStreamSynchronize(st));
-    if(hostCounters[3] != 0) { err = "batched binary tree construction produced an invalid node"; goto fail; }
-
-    // per-mesh box, inflation (1e-5 of the mesh's extent, as a single build) and collapse seed
-    out.boxes.resize(6ull * M);
-    for(uint32_t m = 0; m < M; m++)
-    {
-        const BoxF& b = meshBoxes[m];
-        float ext = 0.0f;
-        for(int k = 0; k < 3; k++)
-        {
-            out.boxes[6ull * m + k] = b.mn[k];
-            out.boxes[6ull * m + 3 + k] = b.mx[k];
-            const float e = fabsf(b.mx[k]) > fabsf(b.mn[k]) ? fabsf(b.mx[k]) : fabsf(b.mn[k]);
-            ext = (ext > e) ? ext : e;
-            const float sp = b.mx[k] - b.mn[k];
-            ext = (ext > sp) ? ext : sp;
-        }
-        segs[m].inflate = ext * 1.0e-5f + 1.0e-30f;
-        seeds[m] = make_uint4(meshRoot[m], m, m, 0u);
-    }
-    MRG_CK(cudaMemcpyAsync(dSegs, segs.data(), sizeof(MeshSeg) * M, cudaMemcpyHostToDevice, st));
-    MRG_CK(cudaMemcpyAsync(dQ[0], seeds.data(), sizeof(uint4) * M, cudaMemcpyHostToDevice, st));
+    if(hostCounters[kCtrError] != 0) { err = "batched binary tree construction produced an invalid node"; goto fail; }
 
     ca.segs = dSegs;
     ca.nodes = dNodes; ca.nodeBoxes = dNodeBoxes; ca.leafBoxes = dLeafBoxes;
     ca.sortedIds = vb.Current(); ca.pos = nullptr; ca.idx = nullptr;
     ca.primKeyBase = 0; ca.kind = 0; ca.maxLeaf = 3; ca.inflate = 0.0f; ca.rawVerts = 0u;
-    ca.wnodes = dW; ca.tris = out.tris; ca.leafIds = nullptr; ca.counters = dCounters;
+    ca.wnodes = dW; ca.tris = tris; ca.leafIds = nullptr; ca.counters = dCounters;
     ca.leafCount = n; ca.wideCap = wideCap;
     ca.costs = dCosts; ca.sahMaxLeaf = sah_max_leaf(false);
-    hostCounters[0] = M; hostCounters[1] = 0; hostCounters[2] = 0; hostCounters[3] = 0;
-    MRG_CK(cudaMemcpyAsync(dCounters, hostCounters, sizeof(hostCounters), cudaMemcpyHostToDevice, st));
-    for(int level = 0; qn > 0; level++)
-    {
-        if(level > 64) { err = "wide BVH deeper than 64 levels"; goto fail; }
-        MRG_CK(cudaMemsetAsync(dCounters + 2, 0, sizeof(uint32_t), st));
-        k_collapse<<<gridFor(qn, 128), 128, 0, st>>>(ca, dQ[cur], qn, dQ[cur ^ 1]);
-        MRG_CK(cudaGetLastError());
-        MRG_CK(cudaMemcpyAsync(hostCounters, dCounters, sizeof(hostCounters), cudaMemcpyDeviceToHost, st));
-        MRG_CK(cudaStreamSynchronize(st));
-        if(hostCounters[3] != 0) { err = "wide BVH collapse reported an invalid tree"; goto fail; }
-        if(hostCounters[0] > wideCap) { err = "wide node capacity exceeded"; goto fail; }
-        qn = hostCounters[2];
-        cur ^= 1;
-    }
-    if(hostCounters[1] != n) { err = "payload count mismatch"; goto fail; }
-    out.nodeCount = hostCounters[0];
-    MRG_CK(cudaMallocAsync(&out.nodes, sizeof(WideNode) * out.nodeCount, st));
-    MRG_CK(cudaMemcpyAsync(out.nodes, dW, sizeof(WideNode) * out.nodeCount, cudaMemcpyDeviceToDevice, st));
+    if(!collapse(ca, dQ, st, hostCounters, err)) goto fail;
+    out.boxes.resize(6ull * M);
+    for(uint32_t m = 0; m < M; m++)
+        for(int k = 0; k < 3; k++)
+        {
+            out.boxes[6ull * m + k] = meshBoxes[m].mn[k];
+            out.boxes[6ull * m + 3 + k] = meshBoxes[m].mx[k];
+        }
+    out.nodes = dW;
+    out.nodeCount = hostCounters[kCtrNodes];
     out.payloadCount = n;
-
-    cudaFreeAsync(dSegs, st); cudaFreeAsync(dFirsts, st); cudaFreeAsync(dCB, st); cudaFreeAsync(dLeafMesh, st);
-    cudaFreeAsync(dLeafBoxes, st); cudaFreeAsync(dCent, st);
-    cudaFreeAsync(dCodes[0], st); cudaFreeAsync(dCodes[1], st);
-    cudaFreeAsync(dIds[0], st); cudaFreeAsync(dIds[1], st); cudaFreeAsync(dTemp, st);
-    cudaFreeAsync(dNodes, st); cudaFreeAsync(dNodeBoxes, st); cudaFreeAsync(dLeafParent, st);
-    cudaFreeAsync(dCnt, st); cudaFreeAsync(dQ[0], st); cudaFreeAsync(dQ[1], st);
-    cudaFreeAsync(dCounters, st); cudaFreeAsync(dMeshRoot, st); cudaFreeAsync(dMeshBoxes, st); cudaFreeAsync(dW, st);
-    cudaFreeAsync(dCosts, st);
-    if(cudaStreamSynchronize(st) != cudaSuccess) { err = "stream sync failed"; return false; }
     return true;
 
 fail:
     cudaStreamSynchronize(st);
-    cudaFree(dSegs); cudaFree(dFirsts); cudaFree(dCB); cudaFree(dLeafMesh);
-    cudaFree(dLeafBoxes); cudaFree(dCent); cudaFree(dCodes[0]); cudaFree(dCodes[1]);
-    cudaFree(dIds[0]); cudaFree(dIds[1]); cudaFree(dTemp); cudaFree(dNodes); cudaFree(dNodeBoxes);
-    cudaFree(dLeafParent); cudaFree(dCnt); cudaFree(dQ[0]); cudaFree(dQ[1]); cudaFree(dCounters);
-    cudaFree(dMeshRoot); cudaFree(dMeshBoxes); cudaFree(dW); cudaFree(dCosts); cudaFree(out.nodes); cudaFree(out.tris);
     out = BatchResult{};
     return false;
 }

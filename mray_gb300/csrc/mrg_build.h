@@ -11,6 +11,22 @@ struct WideNode;
 struct TriRecord;
 struct InstRecord;
 
+// Device memory of a build, carved from slabs that the owner keeps between
+// builds (up to kKeepBytes; larger builds give theirs back).  What a build
+// returns lives here until the next reset().
+class BuildWorkspace
+{
+public:
+    static constexpr size_t kKeepBytes = 256u << 20;
+    void        reset();                        // everything handed out is free again
+    cudaError_t take(void** out, size_t bytes); // 256-byte aligned
+    void        trim();                         // frees the slabs if they pass kKeepBytes
+    void        release();
+private:
+    struct Slab { char* mem; size_t cap, used; };
+    std::vector<Slab> slabs_;
+};
+
 struct BuildInput
 {
     int             kind = 0;          // 0: triangles (pos/idx), 1: boxes (TLAS)
@@ -28,13 +44,13 @@ struct BuildResult
 {
     WideNode*   nodes = nullptr;       // device, nodeCount (child bases local to this build)
     uint32_t    nodeCount = 0;
-    TriRecord*  tris = nullptr;        // kind 0: device, payloadCount records
+    TriRecord*  tris = nullptr;        // kind 0: device, payloadCount records (all in the workspace)
     uint32_t*   leafIds = nullptr;     // kind 1: device, payloadCount leaf ids
     uint32_t    payloadCount = 0;
     float       box[6] = { 0, 0, 0, 0, 0, 0 };
 };
 
-bool build_wide_bvh(const BuildInput& in, BuildResult& out, cudaStream_t st, std::string& err);
+bool build_wide_bvh(const BuildInput& in, BuildResult& out, BuildWorkspace& ws, cudaStream_t st, std::string& err);
 
 // Batched BLAS build (the counterpart of MRay's segmented multi-build,
 // Source/Tracer/AcceleratorLBVH.hpp:585-899): every mesh in one pass of
@@ -52,15 +68,15 @@ struct BatchMeshInput
 
 struct BatchResult
 {
-    WideNode*          nodes = nullptr;     // device, nodeCount (child bases local to the batch)
+    WideNode*          nodes = nullptr;     // workspace, nodeCount (child bases local to the batch)
     uint32_t           nodeCount = 0;
-    TriRecord*         tris = nullptr;      // device, payloadCount records
     uint32_t           payloadCount = 0;
     std::vector<float> boxes;               // 6 per mesh: exact root box
 };
 
-bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, BatchResult& out, cudaStream_t st,
-                          std::string& err);
+// The triangle records go straight to `tris` (one per triangle).
+bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, TriRecord* tris, BatchResult& out,
+                          BuildWorkspace& ws, cudaStream_t st, std::string& err);
 bool relocate_nodes(const WideNode* src, WideNode* dst, uint32_t n, uint32_t nodeOff,
                     uint32_t triOff, cudaStream_t st);
 
