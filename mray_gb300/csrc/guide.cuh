@@ -46,6 +46,16 @@ __device__ __forceinline__ float next_float(uint32_t& s)
     return zs_to_float01(r);
 }
 
+// The state after N numbers.
+template<uint32_t N>
+__device__ __forceinline__ uint32_t skip_numbers(uint32_t s)
+{
+    uint32_t mult = 1u, inc = 0u;
+#pragma unroll
+    for(uint32_t i = 0; i < N; i++) { mult *= 747796405u; inc = inc * 747796405u + 2891336453u; }
+    return s * mult + inc;
+}
+
 __device__ __forceinline__ uint64_t expand3_64(uint32_t v)
 {
     uint64_t x = v & 0x1fffffu;
@@ -171,6 +181,8 @@ __device__ __forceinline__ CodeBase code_base(const Grid& g, float3 pos, float3 
     return b;
 }
 
+constexpr uint32_t kCodeNumbers = 6;   // numbers a stochastic code takes: level, 3 position, 2 normal
+
 __device__ __forceinline__ uint64_t gen_code_stochastic(const Grid& g, const CodeBase& b, float3 pos, uint32_t& rng)
 {
     const uint32_t levelMax = required_bits(g.baseDim) - 1u;
@@ -236,25 +248,6 @@ __device__ __forceinline__ uint32_t try_insert(const Grid& g, uint64_t code)
     for(uint32_t i = index;; i = (i + 1u) & g.tableMask)
     {
         const unsigned long long c = *(volatile unsigned long long*)&g.codes[i];
-        if(c == code) return i;
-        if(c == kEmpty)
-        {
-            const unsigned long long old = atomicCAS(&g.codes[i], kEmpty, (unsigned long long)code);
-            if(old == kEmpty) { atomicAdd(g.counter, 1u); return i; }
-            if(old == code) return i;
-        }
-        if(i == ((index - 1u) & g.tableMask)) break;
-    }
-    return kInvalid;
-}
-
-// TryInsertAtomic's probe from slot `index` whose code was already read as c
-// (the entry-limit test done by the caller).
-__device__ __forceinline__ uint32_t insert_from(const Grid& g, uint64_t code, uint32_t index, unsigned long long c)
-{
-    for(uint32_t i = index;; i = (i + 1u) & g.tableMask)
-    {
-        if(i != index) c = *(volatile unsigned long long*)&g.codes[i];
         if(c == code) return i;
         if(c == kEmpty)
         {

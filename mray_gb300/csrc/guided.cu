@@ -146,7 +146,9 @@ k_guide_backprop(GuideGrid G, GuidePaths Q, PtPaths P, PtSceneTables T,
     }
 }
 
-// KCWriteMarkovChains: the lock winners write the chains they carried.
+// KCWriteMarkovChains: the lock winners write the chains they carried, and
+// free their locks for the next bounce (every lock that was bid for has one
+// winner, and a loser finds another's number or a free lock).
 __global__ void __launch_bounds__(kPtTPB)
 k_guide_write_mc(GuideGrid G, GuidePaths Q, PtPaths P, PtSceneTables T,
                  const uint32_t* __restrict__ aliveList, const uint32_t* __restrict__ aliveCount)
@@ -159,6 +161,7 @@ k_guide_write_mc(GuideGrid G, GuidePaths Q, PtPaths P, PtSceneTables T,
         const uint32_t w = Q.lifted[i];
         if(w == guide::kInvalid) continue;
         if(G.lock[w] != i + 1u) continue;
+        G.lock[w] = 0xFFFFFFFFu;
         const float4 a = Q.tmpA[i];
         const float2 b = Q.tmpB[i];
         G.mcA[w] = a;
@@ -168,68 +171,178 @@ k_guide_write_mc(GuideGrid G, GuidePaths Q, PtPaths P, PtSceneTables T,
 }
 
 // A thread's mixture (GaussLobeMixtureSharedT's layout idea,
-// GuidedPTRendererShaders.h:191-214): per lobe its direction, kappa, alpha,
-// weight, code, slot and pdf scratch, one shared-memory word per field, lobe
-// and thread (thread-contiguous, so bank-conflict free).  Kept off the local
-// stack, which spilled to L2 at this occupancy.
-constexpr uint32_t kMixFields = 10;
-constexpr size_t kMixSmem = (size_t)kMixFields * guide::kLobes * kPtTPB * sizeof(float);
-enum : uint32_t { kMxDx = 0, kMxDy, kMxDz, kMxKappa, kMxAlpha, kMxW, kMxCodeLo, kMxCodeHi, kMxSlot, kMxPdf };
+// GuidedPTRendererShaders.h:191-214): the distinct lobes of its eight draws,
+// one shared-memory word per field, lobe and thread (thread-contiguous, so
+// bank-conflict free; on the local stack they spilled to L2).  Word A is the
+// code's low half until the lobe is found and its slot then, B the high half
+// and later the lobe's pdf.
+constexpr int kGuideTPB = 128;
+#ifndef MRG_GUIDE_BLOCKS
+#define MRG_GUIDE_BLOCKS 5
+#endif
+constexpr int kGuideBlocks = MRG_GUIDE_BLOCKS;      // resident blocks per SM
+constexpr uint32_t kMixFields = 8;
+constexpr size_t kMixSmem = (size_t)kMixFields * guide::kLobes * kGuideTPB * sizeof(float);
+enum : uint32_t { kMxDx = 0, kMxDy, kMxDz, kMxKappa, kMxAlpha, kMxW, kMxA, kMxB };
+constexpr uint32_t kNoLobe = 15u;
 
 struct Mix
 {
-    float* p;
-    __device__ __forceinline__ float& f(uint32_t field, uint32_t j) const
+    float*   p;
+    uint32_t map;       // draw j is lobe (map >> 4 j) & 15 (kNoLobe: its code has no slot)
+    uint32_t n;         // distinct lobes
+    float    sumW;      // weights of all draws
+    uint32_t sel;       // the lobe drawn in proportion to the weights, or kNoLobe
+    __device__ __forceinline__ float& f(uint32_t field, uint32_t k) const
     {
-        return p[(field * guide::kLobes + j) * kPtTPB + threadIdx.x];
+        return p[(field * guide::kLobes + k) * kGuideTPB + threadIdx.x];
     }
-    __device__ __forceinline__ uint32_t& u(uint32_t field, uint32_t j) const
+    __device__ __forceinline__ uint32_t& u(uint32_t field, uint32_t k) const
     {
-        return reinterpret_cast<uint32_t&>(f(field, j));
+        return reinterpret_cast<uint32_t&>(f(field, k));
     }
-    __device__ __forceinline__ guide::Lobe lobe(uint32_t j) const
+    __device__ __forceinline__ uint32_t lobe_of(uint32_t j) const { return (map >> (4u * j)) & 15u; }
+    __device__ __forceinline__ guide::Lobe lobe(uint32_t k) const
     {
         guide::Lobe l;
-        l.dir = make_float3(f(kMxDx, j), f(kMxDy, j), f(kMxDz, j));
-        l.kappa = f(kMxKappa, j);
-        l.alpha = f(kMxAlpha, j);
+        l.dir = make_float3(f(kMxDx, k), f(kMxDy, k), f(kMxDz, k));
+        l.kappa = f(kMxKappa, k);
+        l.alpha = f(kMxAlpha, k);
         return l;
-    }
-    __device__ __forceinline__ void set(uint32_t j, const guide::Lobe& l, float w) const
-    {
-        f(kMxDx, j) = l.dir.x; f(kMxDy, j) = l.dir.y; f(kMxDz, j) = l.dir.z;
-        f(kMxKappa, j) = l.kappa; f(kMxAlpha, j) = l.alpha; f(kMxW, j) = w;
-    }
-    __device__ __forceinline__ bool same_code(uint32_t a, uint32_t b) const
-    {
-        return u(kMxCodeLo, a) == u(kMxCodeLo, b) && u(kMxCodeHi, a) == u(kMxCodeHi, b);
     }
 };
 
-// GaussLobeMixtureT::Pdf; a repeated code's lobe pdf is the earlier one's.
-__device__ __noinline__ float mixture_pdf(Mix m, float sumW, float3 d)
+// Draw j's part of GaussLobeMixtureT::LoadStochastic's choice.
+__device__ __forceinline__ void mix_choose(Mix& m, uint32_t k, uint32_t& rng)
 {
-    if(sumW == 0.0f) return 0.0f;
-    float pdf = 0.0f;
+    const float w = m.f(kMxW, k);
+    m.sumW = add(m.sumW, w);
+    const float ratio = (m.sumW != 0.0f) ? __fdiv_rn(w, m.sumW) : 1.0f;
+    if(guide::next_float(rng) < ratio) m.sel = k;
+}
+
+// The draws of a vertex some of whose codes found no slot (the table is past
+// its entry limit, which ends every later insertion too): a draw without a
+// slot takes no choice number, so the numbers of the draws after it move.
+// Draws up to the first such one stand; a later draw counts if it repeats one
+// of them.
+__device__ __noinline__ void mix_past_limit(const guide::Grid& G, Mix& m, const guide::CodeBase& cb, float3 pos,
+                                            uint32_t& rng)
+{
+    uint64_t code[guide::kLobes];
+    const uint32_t found = m.map;
+    uint32_t map = 0u;
+    bool full = false;
+    m.sumW = 0.0f;
+    m.sel = kNoLobe;
+    for(uint32_t j = 0; j < guide::kLobes; j++)
+    {
+        code[j] = guide::gen_code_stochastic(G, cb, pos, rng);
+        uint32_t k = kNoLobe;
+        if(!full)
+        {
+            k = (found >> (4u * j)) & 15u;
+            if(m.u(kMxA, k) == guide::kInvalid) { k = kNoLobe; full = true; }
+        }
+        else
+            for(uint32_t q = 0; q < j && k == kNoLobe; q++)
+                if(code[q] == code[j]) k = (map >> (4u * q)) & 15u;
+        map |= k << (4u * j);
+        if(k != kNoLobe) mix_choose(m, k, rng);
+    }
+    m.map = map;
+}
+
+// GaussLobeMixtureT::LoadStochastic, in steps that keep the warp's lanes
+// together: all eight codes first (assuming that each finds a slot, the
+// choice numbers between them are only skipped), then a lobe per distinct
+// code, then the choices.  A chain of weight 0 adds nothing to any pdf and is
+// never sampled, so its lobe is not formed.  Drawing, inserting and choosing
+// code by code took 1,879 us of a 256 x 256 x 16 spp frame from an empty grid;
+// 1,535 us now (5 blocks of 128 threads an SM; 4 or 6 are within 1%).
+__device__ __forceinline__ void mix_load(const guide::Grid& G, Mix& m, const guide::CodeBase& cb, float3 pos,
+                                         uint32_t& rng)
+{
+    const uint32_t start = rng;
+    m.map = 0u;
+    m.n = 0u;
 #pragma unroll 1
     for(uint32_t j = 0; j < guide::kLobes; j++)
     {
-        const float w = m.f(kMxW, j);
-        if(w == 0.0f) continue;
-        uint32_t q = 0;
-        while(q < j && !m.same_code(q, j)) q++;
-        const float lp = (q < j) ? m.f(kMxPdf, q) : guide::lobe_pdf(m.lobe(j), d);
-        m.f(kMxPdf, j) = lp;
-        pdf = add(pdf, mul(w, lp));
+        const uint64_t code = guide::gen_code_stochastic(G, cb, pos, rng);
+        rng = guide::skip_numbers<1>(rng);
+        const uint32_t lo = (uint32_t)code, hi = (uint32_t)(code >> 32);
+        uint32_t k = 0;
+        while(k < m.n && (m.u(kMxA, k) != lo || m.u(kMxB, k) != hi)) k++;
+        if(k == m.n)
+        {
+            m.u(kMxA, k) = lo;
+            m.u(kMxB, k) = hi;
+            m.n++;
+        }
+        m.map |= k << (4u * j);
     }
-    return __fdiv_rn(pdf, sumW);
+    bool all = true;
+#pragma unroll 1
+    for(uint32_t k = 0; k < m.n; k++)
+    {
+        const uint32_t slot = guide::try_insert(G, (uint64_t)m.u(kMxA, k) | ((uint64_t)m.u(kMxB, k) << 32));
+        float w = 0.0f;
+        if(slot == guide::kInvalid) all = false;
+        else
+        {
+            w = G.mcW[slot];
+            if(w != 0.0f)
+            {
+                guide::Chain c;
+                const float4 a = G.mcA[slot];
+                c.target = f3(a);
+                c.cosine = a.w;
+                c.weight = w;
+                const guide::Lobe l = guide::chain_to_lobe(c, G.mcN[slot], pos);
+                m.f(kMxDx, k) = l.dir.x; m.f(kMxDy, k) = l.dir.y; m.f(kMxDz, k) = l.dir.z;
+                m.f(kMxKappa, k) = l.kappa; m.f(kMxAlpha, k) = l.alpha;
+            }
+        }
+        m.f(kMxW, k) = w;
+        m.u(kMxA, k) = slot;
+    }
+    rng = start;
+    if(!all) { mix_past_limit(G, m, cb, pos, rng); return; }
+    m.sumW = 0.0f;
+    m.sel = kNoLobe;
+#pragma unroll 1
+    for(uint32_t j = 0; j < guide::kLobes; j++)
+    {
+        rng = guide::skip_numbers<guide::kCodeNumbers>(rng);
+        mix_choose(m, m.lobe_of(j), rng);
+    }
+}
+
+// GaussLobeMixtureT::Pdf, a lobe's pdf once however often it was drawn.
+__device__ __noinline__ float mixture_pdf(Mix m, float3 d)
+{
+    if(m.sumW == 0.0f) return 0.0f;
+#pragma unroll 1
+    for(uint32_t k = 0; k < m.n; k++)
+        if(m.f(kMxW, k) != 0.0f) m.f(kMxB, k) = guide::lobe_pdf(m.lobe(k), d);
+    float pdf = 0.0f;
+#pragma unroll
+    for(uint32_t j = 0; j < guide::kLobes; j++)
+    {
+        const uint32_t k = m.lobe_of(j);
+        if(k == kNoLobe) continue;
+        const float w = m.f(kMxW, k);
+        if(w != 0.0f) pdf = add(pdf, mul(w, m.f(kMxB, k)));
+    }
+    return __fdiv_rn(pdf, m.sumW);
 }
 
 // ---------------------------------------------------------------------------
 // Shade (WorkFunction / LightWorkFunction of the guided renderer).
 // ---------------------------------------------------------------------------
 template<bool SPEC>
-__global__ void __launch_bounds__(kPtTPB)
+__global__ void __launch_bounds__(kGuideTPB, kGuideBlocks)
 k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T, PtWork W,
                uint32_t* nextList, uint32_t* nextCount, uint32_t* shadowCount)
 {
@@ -326,56 +439,13 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                 const float3 woW = normalize3(wo);
 
                 // ---- GaussLobeMixtureT::LoadStochastic ----
-                // A code drawn again gives the slot and lobe it gave before
-                // (nothing writes chains while paths shade), so repeats reuse them.
-                const Mix mx{ gmix };
-                float sumW = 0.0f;
-                uint32_t sIdx = guide::kInvalid;
+                Mix mx;
+                mx.p = gmix;
                 uint32_t rng = Q.bk[i];
-                const float3 codeN = normalize3(woW);
-                const guide::CodeBase cb = guide::code_base(G, pos, codeN);
-#pragma unroll 1
-                for(uint32_t j = 0; j < guide::kLobes; j++)
-                {
-                    const uint64_t code = guide::gen_code_stochastic(G, cb, pos, rng);
-                    mx.u(kMxCodeLo, j) = (uint32_t)code;
-                    mx.u(kMxCodeHi, j) = (uint32_t)(code >> 32);
-                    uint32_t q = 0;
-                    while(q < j && !mx.same_code(q, j)) q++;
-                    uint32_t slot;
-                    float w;
-                    if(q < j)
-                    {
-                        slot = mx.u(kMxSlot, q);
-                        w = mx.f(kMxW, q);
-                        mx.set(j, mx.lobe(q), w);
-                    }
-                    else
-                    {
-                        slot = guide::try_insert(G, code);
-                        guide::Lobe l;
-                        l.dir = make_float3(0, 0, 0); l.kappa = 0.0f; l.alpha = 0.0f;
-                        w = 0.0f;
-                        if(slot != guide::kInvalid)
-                        {
-                            guide::Chain c;
-                            const float4 a = G.mcA[slot];
-                            c.target = f3(a);
-                            c.cosine = a.w;
-                            c.weight = G.mcW[slot];
-                            l = guide::chain_to_lobe(c, G.mcN[slot], pos);
-                            w = c.weight;
-                        }
-                        mx.set(j, l, w);
-                    }
-                    mx.u(kMxSlot, j) = slot;
-                    if(slot == guide::kInvalid) continue;
-                    sumW = add(sumW, w);
-                    const float ratio = (sumW != 0.0f) ? __fdiv_rn(w, sumW) : 1.0f;
-                    if(guide::next_float(rng) < ratio) sIdx = j;
-                }
-                const uint32_t liftedMC = (sIdx != guide::kInvalid) ? mx.u(kMxSlot, sIdx) : guide::kInvalid;
+                mix_load(G, mx, guide::code_base(G, pos, normalize3(woW)), pos, rng);
                 Q.bk[i] = rng;
+                const uint32_t liftedMC = (mx.sel != kNoLobe) ? mx.u(kMxA, mx.sel) : guide::kInvalid;
+                const float selW = (mx.sel != kNoLobe) ? mx.f(kMxW, mx.sel) : 0.0f;
                 const float2 coN = guide::dir_to_conc_octa(woW);
 
                 // ---- mixture or material sample, balance-heuristic pdf ----
@@ -384,7 +454,7 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                 {
                     const float t = fminf(fmaxf(sub(1.0f, specv), 0.0f), 1.0f);
                     mw0 = add(mul(0.0f, sub(1.0f, t)), mul(G.lobeProb, t));     // Math::Lerp(0, p, t)
-                    if(G.fixZeroWeight && (sIdx == guide::kInvalid || mx.f(kMxW, sIdx) == 0.0f)) mw0 = 0.0f;
+                    if(G.fixZeroWeight && selW == 0.0f) mw0 = 0.0f;
                 }
                 const float mw1 = sub(1.0f, mw0);
                 Chan refl;
@@ -397,11 +467,11 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                     // Y axis with pdf 0
                     float3 v = make_float3(0.0f, 1.0f, 0.0f);
                     float mpdf = 0.0f;
-                    if(sIdx != guide::kInvalid && mx.f(kMxW, sIdx) != 0.0f)
+                    if(selW != 0.0f)
                     {
                         const float3 u3 = rnd_s3(L, key, i, depth);
-                        v = guide::lobe_sample(mx.lobe(sIdx), u3.x, u3.y);
-                        mpdf = mixture_pdf(mx, sumW, v);
+                        v = guide::lobe_sample(mx.lobe(mx.sel), u3.x, u3.y);
+                        mpdf = mixture_pdf(mx, v);
                     }
                     wdir = v;
                     const float3 vn = normalize3(v);
@@ -422,7 +492,7 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                                                   add(add(mul(tng.y, Ll.x), mul(btg.y, Ll.y)), mul(nrm.y, Ll.z)),
                                                   add(add(mul(tng.z, Ll.x), mul(btg.z, Ll.y)), mul(nrm.z, Ll.z))));
                     orgOut = pre;
-                    pdf0 = mixture_pdf(mx, sumW, wdir);
+                    pdf0 = mixture_pdf(mx, wdir);
                     pdf1 = bpdf;
                 }
                 const float pdfPath = add(mul(pdf0, mw0), mul(pdf1, mw1));     // BalanceCancelled<2>
@@ -466,7 +536,7 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                     P.prevPdf[i] = pdfPath;
                     P.state[i] = depth | ((isSpec ? 2u : 1u) << 8);
                     Q.prevRefl[i] = __fdiv_rn(avgRefl, fmaxf(pdfPath, 10.0f));
-                    Q.scoreSum[i] = lobeSampled ? sumW : kInf;
+                    Q.scoreSum[i] = lobeSampled ? mx.sumW : kInf;
                     Q.lifted[i] = liftedMC;
                     Q.prevNormal[i] = coN;
                     alive = true;
@@ -486,7 +556,7 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                     const float3 Ls = make_float3(dot3(sdir, tng), dot3(sdir, btg), dot3(sdir, nrm));
                     float bpdf;
                     const Chan srefl = eval_material<NC>(sf, mt, alb, V, Ls, bpdf);
-                    float pdfS = add(mul(mixture_pdf(mx, sumW, sdir), mw0), mul(bpdf, mw1));
+                    float pdfS = add(mul(mixture_pdf(mx, sdir), mw0), mul(bpdf, mw1));
                     pdfS = add(pdfS, lightPdf);
                     Chan srad = chan(0, 0, 0, 0);
                     if(pdfS != 0.0f)
@@ -537,7 +607,7 @@ k_guide_resolve(PtPaths P, GuidePaths Q, const uint32_t* __restrict__ shadowCoun
 __device__ __forceinline__ void ema_terms(uint32_t n0, uint32_t k, float r, float& a, float& b)
 {
     const uint32_t nn = min(n0 + k + 1u, 128u);
-    const float t = fmaxf(__fdiv_rn(1.0f, (float)nn), 0.01f);
+    const float t = (nn >= 100u) ? 0.01f : __fdiv_rn(1.0f, (float)nn);     // max(1 / nn, 0.01)
     a = __fsub_rn(1.0f, t);
     b = __fmul_rn(r, t);
 }
@@ -549,9 +619,10 @@ __device__ __forceinline__ void ema_terms(uint32_t n0, uint32_t k, float r, floa
 // the dependent steps x = x a + b, taking the terms by shuffle.  A cell whose
 // records run past the window goes to the long-run list instead, whole.
 __global__ void __launch_bounds__(kPtTPB)
-k_guide_apply(GuideGrid G, const uint32_t* __restrict__ keys, const float* __restrict__ vals, uint32_t n,
-              uint2* __restrict__ longRuns, uint32_t* longCount)
+k_guide_apply(GuideGrid G, const uint32_t* __restrict__ keys, const float* __restrict__ vals,
+              const uint32_t* __restrict__ count, uint2* __restrict__ longRuns, uint32_t* longCount)
 {
+    const uint32_t n = *count;
     const uint32_t tableSize = G.tableMask + 1u;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -600,63 +671,137 @@ k_guide_apply(GuideGrid G, const uint32_t* __restrict__ keys, const float* __res
     }
 }
 
-// Runs longer than a window, one block per run: the block forms the (a, b)
-// terms of the next 256 records (and whether they are still the run's) into
-// shared memory while thread 0 runs the dependent chain over the previous 256.
-__global__ void __launch_bounds__(kPtTPB)
-k_guide_apply_long(GuideGrid G, const uint32_t* __restrict__ keys, const float* __restrict__ vals, uint32_t n,
-                   const uint2* __restrict__ longRuns, const uint32_t* longCount)
+// Steps [q0, q1) of a long run's chain from v, by one warp: the lanes form the
+// (a, b) terms of 32 records into shared memory while the next 32 values load,
+// lane 0 runs the dependent steps.  Returns lane 0's v.
+struct ChainTerms { float4 a[8], b[8]; };
+__device__ __forceinline__ float chain_steps(const float* __restrict__ vals, uint32_t start, uint32_t q0, uint32_t q1,
+                                             uint32_t n0, float v, ChainTerms& s)
 {
-    __shared__ __align__(16) float sA[2][kPtTPB];
-    __shared__ __align__(16) float sB[2][kPtTPB];
-    const uint32_t runs = *longCount;
-    for(uint32_t e = blockIdx.x; e < runs; e += gridDim.x)
+    const uint32_t lane = threadIdx.x & 31u;
+    float r = (q0 + lane < q1) ? vals[start + q0 + lane] : 0.0f;
+    for(uint32_t q = q0; q < q1; q += 32u)
     {
-        const uint2 run = longRuns[e];
-        const uint32_t start = run.x, cell = run.y;
+        float a = 1.0f, b = 0.0f;
+        if(q + lane < q1) ema_terms(n0, q + lane, r, a, b);
+        reinterpret_cast<float*>(s.a)[lane] = a;
+        reinterpret_cast<float*>(s.b)[lane] = b;
+        __syncwarp();
+        if(q + 32u + lane < q1) r = vals[start + q + 32u + lane];
+        if(lane == 0u)
+        {
+            const uint32_t len = min(32u, q1 - q);
+            if(len == 32u)
+            {
+#pragma unroll
+                for(uint32_t k = 0; k < 8u; k++)
+                {
+                    const float4 a4 = s.a[k], b4 = s.b[k];
+                    v = __fadd_rn(__fmul_rn(v, a4.x), b4.x);
+                    v = __fadd_rn(__fmul_rn(v, a4.y), b4.y);
+                    v = __fadd_rn(__fmul_rn(v, a4.z), b4.z);
+                    v = __fadd_rn(__fmul_rn(v, a4.w), b4.w);
+                }
+            }
+            else
+                for(uint32_t k = 0; k < len; k++)
+                    v = __fadd_rn(__fmul_rn(v, reinterpret_cast<const float*>(s.a)[k]),
+                                  reinterpret_cast<const float*>(s.b)[k]);
+        }
+        __syncwarp();
+    }
+    return v;
+}
+
+// Runs longer than a window: a warp per run of fewer than kLongRun records;
+// the others go to a list of their own.
+constexpr uint32_t kLongRun = 1024;
+__global__ void __launch_bounds__(kPtTPB)
+k_guide_apply_mid(GuideGrid G, const uint32_t* __restrict__ keys, const float* __restrict__ vals,
+                  const uint32_t* __restrict__ count, const uint2* __restrict__ midRuns, const uint32_t* midCount,
+                  uint2* __restrict__ longRuns, uint32_t* longCount)
+{
+    __shared__ ChainTerms terms[kPtTPB / 32];
+    const uint32_t n = *count, runs = *midCount;
+    const uint32_t lane = threadIdx.x & 31u;
+    for(uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < runs; e += gridDim.x * (blockDim.x >> 5))
+    {
+        const uint32_t start = midRuns[e].x, cell = midRuns[e].y;
+        // keys are sorted: the lanes count every 32nd record in the run, then
+        // those of the last 32
+        uint32_t q = start + 32u * lane;
+        const uint32_t in = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, q < n && (keys[q] >> 1) == cell));
+        q = start + 32u * (in - 1u) + lane;
+        const uint32_t len = 32u * (in - 1u) +
+                             (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, q < n && (keys[q] >> 1) == cell));
+        if(len == kLongRun)
+        {
+            if(lane == 0u) longRuns[atomicAdd(longCount, 1u)] = make_uint2(start, cell);
+            continue;
+        }
         const float2 e0 = G.irr[cell];
         const uint32_t n0 = __float_as_uint(e0.y);
-        float v = e0.x;
-        uint32_t total = 0;
-        // terms of chunk ch into buffer ch & 1; returns how many of its records are the run's
-        auto terms = [&](uint32_t ch) -> uint32_t {
-            const uint32_t q = start + ch * kPtTPB + threadIdx.x;
-            const bool in = q < n && (keys[q] >> 1) == cell;
-            float a = 1.0f, b = 0.0f;
-            if(in) ema_terms(n0, q - start, vals[q], a, b);
-            sA[ch & 1u][threadIdx.x] = a;
-            sB[ch & 1u][threadIdx.x] = b;
-            return (uint32_t)__syncthreads_count(in);       // sorted: a prefix of the chunk
-        };
-        uint32_t len = terms(0);
-        for(uint32_t ch = 0;; ch++)
+        const float v = chain_steps(vals, start, 0u, len, n0, e0.x, terms[threadIdx.x >> 5]);
+        if(lane == 0u) G.irr[cell] = make_float2(v, __uint_as_float(min(n0 + len, 128u)));
+    }
+}
+
+// The longest runs, a block each.  The steps x = x a + b depend on one another,
+// 8 cycles each, and a coarse cell takes up to 13k records a bounce.  But a
+// step shrinks a difference in x to at most 0.99 of it, so a chain started
+// anywhere some thousand records early has all but surely reached the true
+// chain's bits: each warp takes an eighth of the run, starts kRunUp records
+// before it, and the value it arrives with is compared bit for bit with where
+// the eighth before it ended.  An eighth whose guess was wrong is run again
+// from the true value, so the result is the sequential one whatever the
+// guesses were.  256 x 256 x 16 spp box, runs above 32 records: 59 us a bounce
+// with a block and one chain each, 44 us with both kernels.
+constexpr uint32_t kRunUp = 2560;
+__global__ void __launch_bounds__(kPtTPB)
+k_guide_apply_long(GuideGrid G, const uint32_t* __restrict__ keys, const float* __restrict__ vals,
+                   const uint32_t* __restrict__ count, const uint2* __restrict__ longRuns, const uint32_t* longCount)
+{
+    constexpr uint32_t kWarps = kPtTPB / 32;
+    __shared__ ChainTerms terms[kWarps];
+    __shared__ float sGuess[kWarps], sEnd[kWarps];
+    const uint32_t n = *count, runs = *longCount;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    for(uint32_t e = blockIdx.x; e < runs; e += gridDim.x)
+    {
+        const uint32_t start = longRuns[e].x, cell = longRuns[e].y;
+        const float2 e0 = G.irr[cell];
+        const uint32_t n0 = __float_as_uint(e0.y);
+        // the run's length: every 64th record, then the last 64
+        uint32_t len = 0;
+        for(bool more = true; more;)
         {
-            const uint32_t cur = ch & 1u;
-            // the next chunk's terms go into the other buffer meanwhile
-            uint32_t next = 0;
-            if(threadIdx.x == 0)
-            {
-                // four terms per shared-memory load, loads unrolled ahead of the chain
-                const float4* A4 = reinterpret_cast<const float4*>(sA[cur]);
-                const float4* B4 = reinterpret_cast<const float4*>(sB[cur]);
-                const uint32_t quads = len >> 2;
-#pragma unroll 8
-                for(uint32_t k = 0; k < quads; k++)
-                {
-                    const float4 a = A4[k], b = B4[k];
-                    v = __fadd_rn(__fmul_rn(v, a.x), b.x);
-                    v = __fadd_rn(__fmul_rn(v, a.y), b.y);
-                    v = __fadd_rn(__fmul_rn(v, a.z), b.z);
-                    v = __fadd_rn(__fmul_rn(v, a.w), b.w);
-                }
-                for(uint32_t k = quads << 2; k < len; k++) v = __fadd_rn(__fmul_rn(v, sA[cur][k]), sB[cur][k]);
-            }
-            total += len;
-            if(len < (uint32_t)kPtTPB) break;           // block-uniform
-            next = terms(ch + 1u);
-            len = next;
+            const uint32_t q = start + len + 64u * threadIdx.x;
+            const uint32_t in = (uint32_t)__syncthreads_count(q < n && (keys[q] >> 1) == cell);
+            more = in == (uint32_t)kPtTPB;
+            len += 64u * in;
         }
-        if(threadIdx.x == 0) G.irr[cell] = make_float2(v, __uint_as_float(min(n0 + total, 128u)));
+        len -= 64u;
+        len += (uint32_t)__syncthreads_count(threadIdx.x < 64u && start + len + threadIdx.x < n &&
+                                             (keys[start + len + threadIdx.x] >> 1) == cell);
+        const uint32_t part = (len + kWarps - 1u) / kWarps;
+        const uint32_t q0 = min(warp * part, len), q1 = min(q0 + part, len);
+        const uint32_t from = q0 - min(q0, kRunUp);        // 0: the true start
+        const float guess = chain_steps(vals, start, from, q0, n0, e0.x, terms[warp]);
+        const float end = chain_steps(vals, start, q0, q1, n0, guess, terms[warp]);
+        if(lane == 0u) { sGuess[warp] = guess; sEnd[warp] = end; }
+        __syncthreads();
+        if(warp == 0u)
+        {
+            float v = sEnd[0];
+            for(uint32_t w = 1; w < kWarps; w++)
+            {
+                if(__float_as_uint(sGuess[w]) == __float_as_uint(v)) v = sEnd[w];
+                else
+                    v = __shfl_sync(0xFFFFFFFFu, chain_steps(vals, start, min(w * part, len),
+                                                             min((w + 1u) * part, len), n0, v, terms[0]), 0);
+            }
+            if(lane == 0u) G.irr[cell] = make_float2(v, __uint_as_float(min(n0 + len, 128u)));
+        }
         __syncthreads();
     }
 }
@@ -693,11 +838,11 @@ cudaError_t guide_shade(const PtLaunch& L, const PtPaths& P, const GuideGrid& G,
         if(e != cudaSuccess) return e;
         attr = true;
     }
-    const unsigned grid = (unsigned)smCount * 2u;
+    const unsigned grid = (unsigned)smCount * kGuideBlocks;
     if(L.spec.enabled)
-        k_shade_guided<true><<<grid, kPtTPB, kMixSmem, st>>>(L, P, G, Q, T, W, nextList, nextCount, shadowCount);
+        k_shade_guided<true><<<grid, kGuideTPB, kMixSmem, st>>>(L, P, G, Q, T, W, nextList, nextCount, shadowCount);
     else
-        k_shade_guided<false><<<grid, kPtTPB, kMixSmem, st>>>(L, P, G, Q, T, W, nextList, nextCount, shadowCount);
+        k_shade_guided<false><<<grid, kGuideTPB, kMixSmem, st>>>(L, P, G, Q, T, W, nextList, nextCount, shadowCount);
     return cudaGetLastError();
 }
 
@@ -713,7 +858,9 @@ cudaError_t guide_apply(const GuideGrid& G, const GuidePaths& Q, int smCount, cu
     const uint32_t n = 2u * Q.slots;
     const uint32_t passes = (Q.keyBits + 7u) / 8u;
     // the records' values ride along as the sort's payload, so the sorted
-    // values are read in order
+    // values are read in order; the first pass leaves the empty records out
+    // and empties the others' keys for the next bounce
+    uint32_t *midCount = Q.longCount, *longCount = Q.longCount + 1, *valid = Q.longCount + 2;
     const uint32_t* kIn = Q.recKey;
     const uint32_t* iIn = reinterpret_cast<const uint32_t*>(Q.recVal);
     for(uint32_t p = 0; p < passes; p++)
@@ -725,19 +872,22 @@ cudaError_t guide_apply(const GuideGrid& G, const GuidePaths& Q, int smCount, cu
         s.dataShift = 0; s.dataWidth = 0;
         s.digitShift = 8u * p;
         s.digitBits = min(8u, Q.keyBits - 8u * p);
-        cudaError_t e = multisplit_pass(kIn, iIn, kOut, iOut, nullptr, n, s, Q.sortHist, st);
+        s.dropEmpty = p == 0u;
+        cudaError_t e = multisplit_pass(kIn, iIn, kOut, iOut, p ? valid : nullptr, n, s, Q.sortHist, st,
+                                        p ? nullptr : Q.recKey, p ? nullptr : valid);
         if(e != cudaSuccess) return e;
         kIn = kOut;
         iIn = iOut;
     }
-    cudaError_t e = cudaMemsetAsync(Q.longCount, 0, sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(Q.longCount, 0, 2 * sizeof(uint32_t), st);
     if(e != cudaSuccess) return e;
     const float* vals = reinterpret_cast<const float*>(iIn);
-    k_guide_apply<<<(unsigned)smCount * 4u, kPtTPB, 0, st>>>(G, kIn, vals, n, Q.longRuns, Q.longCount);
-    k_guide_apply_long<<<(unsigned)smCount * 2u, kPtTPB, 0, st>>>(G, kIn, vals, n, Q.longRuns, Q.longCount);
-    e = cudaGetLastError();
-    if(e != cudaSuccess) return e;
-    return cudaMemsetAsync(Q.recKey, 0xFF, sizeof(uint32_t) * n, st);
+    uint2* longest = Q.longRuns + n / 32u + 1u;
+    k_guide_apply<<<(unsigned)smCount * 4u, kPtTPB, 0, st>>>(G, kIn, vals, valid, Q.longRuns, midCount);
+    k_guide_apply_mid<<<(unsigned)smCount * 4u, kPtTPB, 0, st>>>(G, kIn, vals, valid, Q.longRuns, midCount, longest,
+                                                                 longCount);
+    k_guide_apply_long<<<(unsigned)smCount, kPtTPB, 0, st>>>(G, kIn, vals, valid, longest, longCount);
+    return cudaGetLastError();
 }
 
 } // namespace mrg

@@ -175,6 +175,7 @@ struct mrg_ctx
     mrg::GuidePaths    guideQ{};
     uint32_t           guideCap = 0;              // slots the path state holds
     bool               guideBkValid = false;      // backup streams of (guideBkSeed, W, H, slots)
+    uint32_t           guideSeedSlots = 0;        // start states of (guideBkSeed, W, H) in guideQ.bk0
     uint32_t           guideBkSeed = 0, guideBkW = 0, guideBkH = 0;
 
     // radiance cache (one per context) and its path-tracer buffers

@@ -63,6 +63,7 @@ struct GuideGrid
 struct GuidePaths
 {
     uint32_t* bk;                   // backup RNG state (PermutedCG32)
+    uint32_t* bk0;                  // the states a render starts with
     uint32_t* lifted;               // dLiftedMCIndices
     float*    prevRefl;             // dPrevPathReflectanceOrOutRadiance
     float*    scoreSum;             // dScoreSums
@@ -77,8 +78,9 @@ struct GuidePaths
     uint32_t* sortKeysB;
     uint32_t* sortIdxB;
     uint32_t* sortHist;
-    uint2*    longRuns;             // runs of one cell longer than 32 records: (first position, cell)
-    uint32_t* longCount;
+    uint2*    longRuns;             // runs of one cell past a window of 32 records: (first position, cell);
+                                    // after them those of 1024 records and more
+    uint32_t* longCount;            // both lists' sizes, then the bounce's records
     uint32_t  slots;
     uint32_t  keyBits;              // bits of a record key: log2(table) + 2
 };

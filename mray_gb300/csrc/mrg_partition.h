@@ -15,6 +15,7 @@ struct DigitSpec
     uint32_t batchShift = 0, batchWidth = 0;
     uint32_t dataShift = 0, dataWidth = 0;
     uint32_t digitShift = 0, digitBits = 0;
+    bool     dropEmpty = false;     // keys ~0 are left out (see multisplit_pass)
 };
 
 // Words of the (bucket, tile) count table of one pass.
@@ -27,10 +28,12 @@ inline size_t multi_partition_scratch_words(uint32_t nMax)
 }
 
 // Stable scatter of (key, index) pairs by one digit.  idxIn == nullptr means
-// the element's position.  The count is *nDevice when given, else nMax.
+// the element's position.  The count is *nDevice when given, else nMax.  With
+// spec.dropEmpty the pairs of key ~0 are left out: *nOut is how many remain,
+// and `emptied` (keysIn itself) gets ~0 where a key was taken.
 cudaError_t multisplit_pass(const uint32_t* keysIn, const uint32_t* idxIn, uint32_t* keysOut, uint32_t* idxOut,
                             const uint32_t* nDevice, uint32_t nMax, const DigitSpec& spec, uint32_t* hist,
-                            cudaStream_t st);
+                            cudaStream_t st, uint32_t* emptied = nullptr, uint32_t* nOut = nullptr);
 
 // RayPartitioner::MultiPartition: stable sort by (batch, data) bits, then the
 // start offset and key of every run of equal batch bits.  scratch holds

@@ -5,10 +5,10 @@
 // MRay sorts with CUB's radix sort and finds the splits with a binary
 // partition, waiting on the host in between.  Here one radix digit (up to 8
 // bits, 256 buckets) is one pass of three kernels:
-//   hist     per-tile bucket counts (shared-memory, warp-aggregated atomics)
-//   scan     exclusive scan of the bucket-major (bucket, tile) count table
-//   scatter  stable ranks inside each tile (warp match + per-warp counts in
-//            shared memory), written to the bucket's global offset
+//   hist     per-tile bucket counts (shared-memory atomics) and bucket totals
+//   rows     a block per bucket scans its row of the (bucket, tile) count table
+//   scatter  stable ranks inside each tile (warp match against per-warp counts
+//            in shared memory), written to the bucket's global offset
 // The element count may live in device memory (a path tracer's alive count),
 // so a pass is enqueued without knowing it; the grid is sized for an upper
 // bound and tiles past the count contribute nothing.
@@ -23,6 +23,7 @@ constexpr int kMsItems = 8;
 constexpr int kMsTile = kMsTPB * kMsItems;     // 2048 elements per tile
 constexpr int kMsWarps = kMsTPB / 32;
 constexpr int kScanTPB = 1024;
+constexpr uint32_t kMsEmpty = 0xFFFFFFFFu;      // an empty key (DigitSpec::dropEmpty)
 
 __device__ __forceinline__ uint32_t bits_of(uint32_t v, uint32_t shift, uint32_t width)
 {
@@ -42,9 +43,10 @@ __device__ __forceinline__ uint32_t count_of(const uint32_t* nDevice, uint32_t n
     return nDevice ? *nDevice : nHost;
 }
 
+// Bucket counts of one tile, and their sums over all tiles.
 __global__ void __launch_bounds__(kMsTPB)
 k_ms_hist(const uint32_t* __restrict__ keys, const uint32_t* nDevice, uint32_t nHost, DigitSpec spec,
-          uint32_t* __restrict__ hist, uint32_t numTiles)
+          uint32_t* __restrict__ hist, uint32_t numTiles, uint32_t* __restrict__ totals)
 {
     __shared__ uint32_t sHist[256];
     const uint32_t nb = 1u << spec.digitBits;
@@ -52,52 +54,26 @@ k_ms_hist(const uint32_t* __restrict__ keys, const uint32_t* nDevice, uint32_t n
     __syncthreads();
     const uint32_t n = count_of(nDevice, nHost);
     const uint32_t tileStart = blockIdx.x * (uint32_t)kMsTile;
+    uint32_t key[kMsItems];
+#pragma unroll
     for(int r = 0; r < kMsItems; r++)
     {
         const uint32_t e = tileStart + (uint32_t)r * kMsTPB + threadIdx.x;
-        const bool valid = e < n;
-        const uint32_t d = valid ? digit_of(spec, __ldg(&keys[e])) : 0xFFFFFFFFu;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-        const uint32_t lane = threadIdx.x & 31u;
-        if(valid && (__ffs(peers) - 1) == (int)lane) atomicAdd(&sHist[d], (uint32_t)__popc(peers));
+        key[r] = (e < n) ? __ldg(&keys[e]) : kMsEmpty;
+    }
+#pragma unroll
+    for(int r = 0; r < kMsItems; r++)
+    {
+        const uint32_t e = tileStart + (uint32_t)r * kMsTPB + threadIdx.x;
+        if(e < n && !(spec.dropEmpty && key[r] == kMsEmpty)) atomicAdd(&sHist[digit_of(spec, key[r])], 1u);
     }
     __syncthreads();
-    for(uint32_t b = threadIdx.x; b < nb; b += kMsTPB) hist[(size_t)b * numTiles + blockIdx.x] = sHist[b];
-}
-
-// Exclusive scan of len counts in place; one block (len <= 256 * 2^16).
-__global__ void __launch_bounds__(kScanTPB)
-k_ms_scan(uint32_t* __restrict__ hist, uint32_t len)
-{
-    __shared__ uint32_t sPart[kScanTPB];
-    const uint32_t per = (len + kScanTPB - 1) / kScanTPB;
-    const uint32_t beg = min(len, threadIdx.x * per), end = min(len, beg + per);
-    uint32_t sum = 0;
-    for(uint32_t i = beg; i < end; i++) sum += hist[i];
-    sPart[threadIdx.x] = sum;
-    __syncthreads();
-    // Hillis-Steele inclusive scan of the per-thread sums
-    for(uint32_t off = 1; off < kScanTPB; off <<= 1)
+    for(uint32_t b = threadIdx.x; b < nb; b += kMsTPB)
     {
-        const uint32_t v = (threadIdx.x >= off) ? sPart[threadIdx.x - off] : 0u;
-        __syncthreads();
-        sPart[threadIdx.x] += v;
-        __syncthreads();
-    }
-    uint32_t run = sPart[threadIdx.x] - sum;
-    for(uint32_t i = beg; i < end; i++)
-    {
-        const uint32_t v = hist[i];
-        hist[i] = run;
-        run += v;
+        hist[(size_t)b * numTiles + blockIdx.x] = sHist[b];
+        if(sHist[b]) atomicAdd(&totals[b], sHist[b]);
     }
 }
-
-// Large count tables: a three-kernel scan (per-block sums, one-block scan of
-// the sums, per-block exclusive scan plus its offset), kScanChunk entries per
-// block, 4 per thread.
-constexpr uint32_t kScanChunk = 4u * kScanTPB;
-constexpr uint32_t kSingleBlockScan = 65536u;   // at most this many entries: k_ms_scan
 
 // Exclusive scan of v across the block; the block's total in *total.
 __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total)
@@ -126,98 +102,99 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total)
     }
     __syncthreads();
     const uint32_t before = (warp ? sWarp[warp - 1] : 0u) + x - v;
-    if(total) *total = sWarp[kScanTPB / 32 - 1];
+    *total = sWarp[kScanTPB / 32 - 1];
     __syncthreads();
     return before;
 }
 
+// Output offsets: block b turns bucket b's row of tile counts into positions,
+// from the sum of the buckets before it.  One launch for any table size; a
+// one-block scan, or three kernels over tables past 65,536 counts (6.6 us for
+// 262,144), did this before.
 __global__ void __launch_bounds__(kScanTPB)
-k_scan_sums(const uint32_t* __restrict__ hist, uint32_t len, uint32_t* __restrict__ sums)
+k_ms_rows(uint32_t* __restrict__ hist, uint32_t numTiles, const uint32_t* __restrict__ totals, uint32_t* nOut)
 {
-    const uint32_t base = blockIdx.x * kScanChunk + 4u * threadIdx.x;
-    uint32_t v = 0;
-#pragma unroll
-    for(uint32_t k = 0; k < 4u; k++) v += (base + k < len) ? hist[base + k] : 0u;
-    uint32_t total;
-    block_exclusive(v, &total);
-    if(threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kScanTPB)
-k_scan_top(uint32_t* __restrict__ sums, uint32_t n)
-{
-    uint32_t carry = 0;
-    for(uint32_t b = 0; b < n; b += kScanTPB)
+    const uint32_t b = blockIdx.x;
+    uint32_t carry;
+    block_exclusive(threadIdx.x < b ? totals[threadIdx.x] : 0u, &carry);      // at most 256 buckets
+    if(nOut && b == gridDim.x - 1u && threadIdx.x == 0u) *nOut = carry + totals[b];
+    uint32_t* row = hist + (size_t)b * numTiles;
+    for(uint32_t t = 0; t < numTiles; t += kScanTPB)
     {
-        const uint32_t i = b + threadIdx.x;
-        const uint32_t v = (i < n) ? sums[i] : 0u;
+        const uint32_t i = t + threadIdx.x;
+        const uint32_t v = (i < numTiles) ? row[i] : 0u;
         uint32_t total;
-        const uint32_t ex = block_exclusive(v, &total);
-        if(i < n) sums[i] = carry + ex;
+        const uint32_t before = block_exclusive(v, &total);
+        if(i < numTiles) row[i] = carry + before;
         carry += total;
     }
 }
 
-__global__ void __launch_bounds__(kScanTPB)
-k_scan_apply(uint32_t* __restrict__ hist, uint32_t len, const uint32_t* __restrict__ sums)
-{
-    const uint32_t base = blockIdx.x * kScanChunk + 4u * threadIdx.x;
-    uint32_t a[4];
-#pragma unroll
-    for(uint32_t k = 0; k < 4u; k++) a[k] = (base + k < len) ? hist[base + k] : 0u;
-    uint32_t run = sums[blockIdx.x] + block_exclusive(a[0] + a[1] + a[2] + a[3], nullptr);
-#pragma unroll
-    for(uint32_t k = 0; k < 4u; k++)
-        if(base + k < len) { hist[base + k] = run; run += a[k]; }
-}
-
+// Stable scatter of one tile.  Each warp takes 256 consecutive elements and
+// ranks them against its own counters (no block barrier), one pass over the
+// buckets turns the eight warps' counts into output positions, and every
+// element goes to its position.  Bound by latency and the scattered writes:
+// 2.1M elements, 8 bits, in 9.0 us; ranking 256 elements of the whole
+// block at a time, with four barriers each, took 17.8 us.
 __global__ void __launch_bounds__(kMsTPB)
-k_ms_scatter(const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ idxIn,
+k_ms_scatter(const uint32_t* keysIn, const uint32_t* __restrict__ idxIn,
              uint32_t* __restrict__ keysOut, uint32_t* __restrict__ idxOut,
              const uint32_t* nDevice, uint32_t nHost, DigitSpec spec,
-             const uint32_t* __restrict__ hist, uint32_t numTiles)
+             const uint32_t* __restrict__ hist, uint32_t numTiles, uint32_t* emptied)
 {
-    __shared__ uint32_t sBase[256];
-    __shared__ uint32_t sWarp[kMsWarps][256];
+    __shared__ uint32_t sCount[kMsWarps][256];
     const uint32_t nb = 1u << spec.digitBits;
     const uint32_t n = count_of(nDevice, nHost);
     const uint32_t tileStart = blockIdx.x * (uint32_t)kMsTile;
     if(tileStart >= n) return;                              // block-uniform
-    for(uint32_t b = threadIdx.x; b < nb; b += kMsTPB) sBase[b] = hist[(size_t)b * numTiles + blockIdx.x];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lowerMask = (1u << lane) - 1u;
+    for(uint32_t b = lane; b < nb; b += 32u) sCount[warp][b] = 0u;
+    __syncwarp();
+    const uint32_t first = tileStart + warp * (uint32_t)(kMsTile / kMsWarps);
+    uint32_t key[kMsItems], digit[kMsItems], rank[kMsItems];
+#pragma unroll
     for(int r = 0; r < kMsItems; r++)
     {
-        for(uint32_t i = threadIdx.x; i < (uint32_t)kMsWarps * nb; i += kMsTPB) sWarp[i / nb][i % nb] = 0u;
-        __syncthreads();
-        const uint32_t e = tileStart + (uint32_t)r * kMsTPB + threadIdx.x;
-        const bool valid = e < n;
-        uint32_t key = 0, idx = 0, d = 0xFFFFFFFFu;
-        if(valid)
-        {
-            key = keysIn[e];
-            idx = idxIn ? idxIn[e] : e;
-            d = digit_of(spec, key);
-        }
+        const uint32_t e = first + (uint32_t)r * 32u + lane;
+        key[r] = (e < n) ? keysIn[e] : kMsEmpty;
+    }
+#pragma unroll
+    for(int r = 0; r < kMsItems; r++)
+    {
+        const uint32_t e = first + (uint32_t)r * 32u + lane;
+        const bool valid = e < n && !(spec.dropEmpty && key[r] == kMsEmpty);
+        const uint32_t d = valid ? digit_of(spec, key[r]) : 0xFFFFFFFFu;
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-        const uint32_t rank = (uint32_t)__popc(peers & lowerMask);
-        if(valid && rank == 0u) sWarp[warp][d] = (uint32_t)__popc(peers);
-        __syncthreads();
-        if(valid)
+        const uint32_t before = valid ? sCount[warp][d] : 0u;
+        __syncwarp();
+        if(valid && (peers & lowerMask) == 0u) sCount[warp][d] = before + (uint32_t)__popc(peers);
+        __syncwarp();
+        digit[r] = d;
+        rank[r] = before + (uint32_t)__popc(peers & lowerMask);
+        if(spec.dropEmpty && valid) emptied[e] = kMsEmpty;
+    }
+    __syncthreads();
+    for(uint32_t b = threadIdx.x; b < nb; b += kMsTPB)
+    {
+        uint32_t at = hist[(size_t)b * numTiles + blockIdx.x];
+#pragma unroll
+        for(int w = 0; w < kMsWarps; w++)
         {
-            uint32_t pos = sBase[d] + rank;
-            for(uint32_t w = 0; w < warp; w++) pos += sWarp[w][d];
-            keysOut[pos] = key;
-            idxOut[pos] = idx;
+            const uint32_t c = sCount[w][b];
+            sCount[w][b] = at;
+            at += c;
         }
-        __syncthreads();
-        for(uint32_t b = threadIdx.x; b < nb; b += kMsTPB)
-        {
-            uint32_t t = 0;
-            for(int w = 0; w < kMsWarps; w++) t += sWarp[w][b];
-            sBase[b] += t;
-        }
-        __syncthreads();
+    }
+    __syncthreads();
+#pragma unroll
+    for(int r = 0; r < kMsItems; r++)
+    {
+        if(digit[r] == 0xFFFFFFFFu) continue;
+        const uint32_t e = first + (uint32_t)r * 32u + lane;
+        const uint32_t pos = sCount[warp][digit[r]] + rank[r];
+        keysOut[pos] = key[r];
+        idxOut[pos] = idxIn ? idxIn[e] : e;
     }
 }
 
@@ -317,30 +294,25 @@ cudaError_t ray_coherence_order(const void* rays, const uint32_t* idx, uint32_t 
 size_t multisplit_hist_words(uint32_t nMax, uint32_t digitBits)
 {
     const uint32_t tiles = (nMax + kMsTile - 1) / kMsTile;
-    const size_t len = (size_t)(tiles ? tiles : 1u) << digitBits;
-    // the count table, then the block sums of its scan
-    return len + (len + kScanChunk - 1) / kScanChunk;
+    // the count table, then the bucket totals
+    return ((size_t)(tiles ? tiles : 1u) << digitBits) + 256u;
 }
 
 cudaError_t multisplit_pass(const uint32_t* keysIn, const uint32_t* idxIn, uint32_t* keysOut, uint32_t* idxOut,
                             const uint32_t* nDevice, uint32_t nMax, const DigitSpec& spec, uint32_t* hist,
-                            cudaStream_t st)
+                            cudaStream_t st, uint32_t* emptied, uint32_t* nOut)
 {
+    if(spec.dropEmpty && (!emptied || !nOut)) return cudaErrorInvalidValue;
     if(spec.digitBits == 0 || spec.digitBits > 8) return cudaErrorInvalidValue;
     uint32_t tiles = (nMax + kMsTile - 1) / kMsTile;
     if(tiles == 0) tiles = 1;
-    const uint32_t len = tiles << spec.digitBits;
-    k_ms_hist<<<tiles, kMsTPB, 0, st>>>(keysIn, nDevice, nMax, spec, hist, tiles);
-    if(len <= kSingleBlockScan) k_ms_scan<<<1, kScanTPB, 0, st>>>(hist, len);
-    else
-    {
-        const uint32_t blocks = (len + kScanChunk - 1) / kScanChunk;
-        uint32_t* sums = hist + len;
-        k_scan_sums<<<blocks, kScanTPB, 0, st>>>(hist, len, sums);
-        k_scan_top<<<1, kScanTPB, 0, st>>>(sums, blocks);
-        k_scan_apply<<<blocks, kScanTPB, 0, st>>>(hist, len, sums);
-    }
-    k_ms_scatter<<<tiles, kMsTPB, 0, st>>>(keysIn, idxIn, keysOut, idxOut, nDevice, nMax, spec, hist, tiles);
+    const uint32_t nb = 1u << spec.digitBits;
+    uint32_t* totals = hist + ((size_t)tiles << spec.digitBits);
+    cudaError_t e = cudaMemsetAsync(totals, 0, sizeof(uint32_t) * nb, st);
+    if(e != cudaSuccess) return e;
+    k_ms_hist<<<tiles, kMsTPB, 0, st>>>(keysIn, nDevice, nMax, spec, hist, tiles, totals);
+    k_ms_rows<<<nb, kScanTPB, 0, st>>>(hist, tiles, totals, nOut);
+    k_ms_scatter<<<tiles, kMsTPB, 0, st>>>(keysIn, idxIn, keysOut, idxOut, nDevice, nMax, spec, hist, tiles, emptied);
     return cudaGetLastError();
 }
 

@@ -4,6 +4,7 @@
 #include "mrg_ctx.h"
 #include "zsobol.cuh"
 #include "host_math.h"
+#include "mrg_mt19937.h"
 
 #include <cuda_runtime.h>
 
@@ -11,7 +12,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <random>
 #include <string>
 #include <vector>
 
@@ -205,7 +205,7 @@ mrg_status env_prepare(mrg_ctx* c)
 // per-pixel seeds of (width, height, seed), kept while those stay the same.
 // Both groups seed a pixel from the same std::mt19937 output
 // (RNGGroupZSobol, Random.cu:1175-1200; RNGGroupIndependent, Random.cu:683-704).
-mrg_status pt_zsobol(mrg_ctx* c, const mrg_pt_params& p, mrg::PtLaunch& L, const std::string& w)
+mrg_status pt_zsobol(mrg_ctx* c, const mrg_pt_params& p, mrg::PtLaunch& L, cudaStream_t st, const std::string& w)
 {
     if(!c->dZsTables)
     {
@@ -216,14 +216,11 @@ mrg_status pt_zsobol(mrg_ctx* c, const mrg_pt_params& p, mrg::PtLaunch& L, const
     }
     if(!c->dZsSeeds || c->zsW != p.width || c->zsH != p.height || c->zsSeed != p.seed)
     {
-        std::vector<uint32_t> seeds((size_t)p.width * p.height);
-        mrg_status s = mrg_zsobol_seeds(p.width, p.height, p.seed, seeds.data());
-        if(s != MRG_OK) return s;
+        const uint64_t n = (uint64_t)p.width * p.height;
         cudaFree(c->dZsSeeds);
         c->dZsSeeds = nullptr;
-        PT_TRY(cudaMalloc(&c->dZsSeeds, sizeof(uint32_t) * seeds.size()), "ZSobol seeds");
-        PT_TRY(cudaMemcpy(c->dZsSeeds, seeds.data(), sizeof(uint32_t) * seeds.size(), cudaMemcpyHostToDevice),
-               "ZSobol seeds");
+        PT_TRY(cudaMalloc(&c->dZsSeeds, sizeof(uint32_t) * n), "ZSobol seeds");
+        PT_TRY(mrg::mt19937_outputs(p.seed, 0, (uint32_t)n, false, c->dZsSeeds, st), "ZSobol seeds");
         c->zsW = p.width; c->zsH = p.height; c->zsSeed = p.seed;
     }
     const uint64_t maxSpp = p.samplerMaxSpp ? p.samplerMaxSpp : (uint64_t)p.sampleStart + p.spp;
@@ -714,7 +711,7 @@ struct PtRun
     uint32_t            slots = 0;
 };
 
-mrg_status pt_setup(mrg_ctx* c, const mrg_pt_params* p, PtRun& R, const char* who)
+mrg_status pt_setup(mrg_ctx* c, const mrg_pt_params* p, PtRun& R, cudaStream_t st, const char* who)
 {
     const std::string w(who);
     if(!c->built) return mrg::set_error(MRG_ERR_NOT_BUILT, w + ": call mrg_build first");
@@ -754,7 +751,7 @@ mrg_status pt_setup(mrg_ctx* c, const mrg_pt_params* p, PtRun& R, const char* wh
        ((uint64_t)p->sampleStart + p->spp) * ((uint64_t)p->maxDepth + 1u) * 16u > 0x100000000ull)
         return mrg::set_error(MRG_ERR_INVALID_ARG, w + ": samples x depth exceed the PCG32 stream");
     L.sampler = p->sampler;
-    if(L.sampler != MRG_PT_SAMPLER_INDEPENDENT && (s = pt_zsobol(c, *p, L, w)) != MRG_OK) return s;
+    if(L.sampler != MRG_PT_SAMPLER_INDEPENDENT && (s = pt_zsobol(c, *p, L, st, w)) != MRG_OK) return s;
     camera_frame(*p, L.cam);
     // Auto: group the paths by work where several kinds of work can occur and
     // the pass is large enough for coherent shading to pay for the grouping.
@@ -962,7 +959,7 @@ mrg_status mrg_pt_render(mrg_ctx* c, const mrg_pt_params* p, float* dImage, void
     if(!c || !p || !dImage) return mrg::set_error(MRG_ERR_INVALID_ARG, "mrg_pt_render: null pointer");
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, "mrg_pt_render");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render");
     if(s != MRG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     PtLane lanes[2];
@@ -994,7 +991,7 @@ mrg_status mrg_pt_render_cached(mrg_ctx* c, const mrg_pt_params* p, float* dImag
     constexpr uint32_t kRec = 2;
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, "mrg_pt_render_cached");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render_cached");
     if(s != MRG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // buffers: query in / out / list, per-slot training records, batch, counters
@@ -1079,7 +1076,7 @@ mrg_status mrg_pt_adjoint(mrg_ctx* c, const mrg_pt_params* p, uint32_t texId, co
             return mrg::set_error(MRG_ERR_INVALID_ARG, "mrg_pt_adjoint: the parameter texture must feed Lambert albedos");
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, "mrg_pt_adjoint");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_adjoint");
     if(s != MRG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     mrg::PtAdjoint& A = R.L.adj;
@@ -1217,6 +1214,7 @@ mrg_status guide_clear(mrg_ctx* c)
     PT_TRY(cudaMemset(G.mcW, 0, sizeof(float) * T), "mrg_guide: clear");
     PT_TRY(cudaMemset(G.mcN, 0, sizeof(uint32_t) * T), "mrg_guide: clear");
     PT_TRY(cudaMemset(G.irr, 0, sizeof(float2) * T), "mrg_guide: clear");
+    PT_TRY(cudaMemset(G.lock, 0xFF, sizeof(uint32_t) * T), "mrg_guide: clear");
     c->guideCamSet = false;
     c->guideBkValid = false;
     return MRG_OK;
@@ -1236,9 +1234,9 @@ mrg_status guide_paths(mrg_ctx* c, uint32_t slots)
         c->guideCap = 0;
         Q = mrg::GuidePaths{};
         const size_t n = slots;
-        const size_t sizes[17] = { n * 4, n * 4, n * 4, n * 4, n * 8, n * 4, n * 16, n * 8, n * 8, n * 8,
+        const size_t sizes[18] = { n * 4, n * 4, n * 4, n * 4, n * 4, n * 8, n * 4, n * 16, n * 8, n * 8, n * 8,
                                    n * 8, n * 8, n * 8, n * 8, 4 * mrg::multisplit_hist_words(2u * slots, 8),
-                                   8 * ((2 * n) / 32 + 1), 4 };
+                                   8 * ((2 * n) / 32 + 1 + (2 * n) / 1024 + 1), 16 };
         size_t need = 0;
         for(size_t sz : sizes) need += (sz + 255) & ~size_t(255);
         char* base = nullptr;
@@ -1248,6 +1246,7 @@ mrg_status guide_paths(mrg_ctx* c, uint32_t slots)
         int k = 0;
         auto take = [&]() { char* q = base + off; off += (sizes[k++] + 255) & ~size_t(255); return q; };
         Q.bk = reinterpret_cast<uint32_t*>(take());
+        Q.bk0 = reinterpret_cast<uint32_t*>(take());
         Q.lifted = reinterpret_cast<uint32_t*>(take());
         Q.prevRefl = reinterpret_cast<float*>(take());
         Q.scoreSum = reinterpret_cast<float*>(take());
@@ -1266,6 +1265,7 @@ mrg_status guide_paths(mrg_ctx* c, uint32_t slots)
         Q.longCount = reinterpret_cast<uint32_t*>(take());
         c->guideCap = slots;
         c->guideBkValid = false;
+        c->guideSeedSlots = 0;
         // every bounce leaves the records empty again (guide_apply)
         PT_TRY(cudaMemset(Q.recKey, 0xFF, sizeof(uint32_t) * 2u * n), "mrg_pt_render_guided: records");
     }
@@ -1278,21 +1278,24 @@ mrg_status guide_paths(mrg_ctx* c, uint32_t slots)
 // Backup streams: slot i starts at PermutedCG32::GenerateState of output
 // width * height + i of std::mt19937(seed) (the outputs before it seed the
 // pixels' main streams, as RNGGroupIndependent::Seed orders them,
-// Random.cu:683-724).
-mrg_status guide_backup_streams(mrg_ctx* c, const mrg_pt_params* p, uint32_t slots)
+// Random.cu:683-724).  The start states of (width, height, seed) are kept, as
+// the pixels' seeds are (pt_zsobol): a cleared grid begins with them again.
+mrg_status guide_backup_streams(mrg_ctx* c, const mrg_pt_params* p, uint32_t slots, cudaStream_t st)
 {
-    if(c->guideBkValid && c->guideBkSeed == p->seed && c->guideBkW == p->width && c->guideBkH == p->height)
-        return MRG_OK;
-    PT_TRY(cudaDeviceSynchronize(), "mrg_pt_render_guided: earlier work");
-    std::mt19937 rng(p->seed);
-    rng.discard((unsigned long long)p->width * p->height);
-    std::vector<uint32_t> st(slots);
-    for(uint32_t i = 0; i < slots; i++)
-        st[i] = ((uint32_t)rng() + mrg::kBackupPcgInc) * mrg::kBackupPcgMult + mrg::kBackupPcgInc;
-    PT_TRY(cudaMemcpy(c->guideQ.bk, st.data(), sizeof(uint32_t) * slots, cudaMemcpyHostToDevice),
+    const bool same = c->guideSeedSlots == slots && c->guideBkSeed == p->seed && c->guideBkW == p->width &&
+                      c->guideBkH == p->height;
+    if(same && c->guideBkValid) return MRG_OK;
+    if(!same)
+    {
+        c->guideSeedSlots = 0;
+        PT_TRY(mrg::mt19937_outputs(p->seed, (uint64_t)p->width * p->height, slots, true, c->guideQ.bk0, st),
+               "mrg_pt_render_guided: backup streams");
+        c->guideSeedSlots = slots;
+        c->guideBkSeed = p->seed; c->guideBkW = p->width; c->guideBkH = p->height;
+    }
+    PT_TRY(cudaMemcpyAsync(c->guideQ.bk, c->guideQ.bk0, sizeof(uint32_t) * (size_t)slots, cudaMemcpyDeviceToDevice, st),
            "mrg_pt_render_guided: backup streams");
     c->guideBkValid = true;
-    c->guideBkSeed = p->seed; c->guideBkW = p->width; c->guideBkH = p->height;
     return MRG_OK;
 }
 
@@ -1308,16 +1311,13 @@ cudaError_t guided_bounces(mrg_ctx* c, PtRun& R, const PtLane& lane)
     const mrg::GuidePaths& Q = c->guideQ;
     cudaStream_t st = lane.st, side = lane.side;
     const bool overlap = side != st;
-    const size_t T = (size_t)G.tableMask + 1u;
     cudaError_t e = mrg::pt_raygen(L, P, P.listA, c->smCount, st);
     if(e == cudaSuccess) e = cudaMemsetAsync(Q.lifted, 0xFF, sizeof(uint32_t) * (size_t)R.slots, st);
     for(uint32_t depth = 0; depth < L.maxDepth && e == cudaSuccess; depth++)
     {
         const PtBounce B(P, R.scr, depth, R.partition);
         const uint32_t* aliveCount = B.ctr + mrg::kCtrAlive;
-        e = cudaMemsetAsync(G.lock, 0xFF, sizeof(uint32_t) * T, st);
-        if(e == cudaSuccess)
-            e = mrg::launch_closest(c->scene, B.closest, P.rays, B.alive, 0, P.hits, P.meta, c->smCount, st, aliveCount);
+        e = mrg::launch_closest(c->scene, B.closest, P.rays, B.alive, 0, P.hits, P.meta, c->smCount, st, aliveCount);
         if(e == cudaSuccess && R.partition)
             e = mrg::pt_group(L, P, R.T.surfaces, R.T.nSurfaces, B.alive, B.ctr, st);
         if(e == cudaSuccess && overlap && depth > 0) e = cudaStreamWaitEvent(st, lane.evResolved, 0);
@@ -1420,6 +1420,7 @@ mrg_status mrg_guide_destroy(mrg_ctx* c)
     c->dGuideGrid = nullptr;
     c->dGuidePaths = nullptr;
     c->guideCap = 0;
+    c->guideSeedSlots = 0;
     c->guideQ = mrg::GuidePaths{};
     c->guide = mrg::GuideGrid{};
     c->guideOn = false;
@@ -1483,10 +1484,10 @@ mrg_status mrg_pt_render_guided(mrg_ctx* c, const mrg_pt_params* p, float* dImag
         return mrg::set_error(MRG_ERR_INVALID_ARG, "mrg_pt_render_guided: samplers INDEPENDENT and PCG32 only");
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, "mrg_pt_render_guided");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render_guided");
     if(s != MRG_OK) return s;
     if((s = guide_paths(c, R.slots)) != MRG_OK) return s;
-    if((s = guide_backup_streams(c, p, R.slots)) != MRG_OK) return s;
+    if((s = guide_backup_streams(c, p, R.slots, static_cast<cudaStream_t>(stream))) != MRG_OK) return s;
     if(!c->guideCamSet)
     {
         // GenCameraPosition of the pinhole camera: its position
