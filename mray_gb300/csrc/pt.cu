@@ -39,8 +39,9 @@ k_raygen(PtLaunch L, PtPaths P, uint32_t* aliveList)
         const uint32_t pixel = slot_pixel(L, i);
         const uint32_t x = pixel % L.width, y = pixel / L.width;
         const uint32_t key = path_key(L.seed, pixel, slot_sample(L, i));
-        const float ox = gaussian_offset(rnd_s(L, key, i, 0, 6), L.filterSigma);
-        const float oy = gaussian_offset(rnd_s(L, key, i, 0, 7), L.filterSigma);
+        const float2 xi = rnd_s67(L, key, i);
+        const float ox = gaussian_offset(xi.x, L.filterSigma);
+        const float oy = gaussian_offset(xi.y, L.filterSigma);
         const float dx = __fdiv_rn(L.cam.planeSize[0], (float)L.width);
         const float dy = __fdiv_rn(L.cam.planeSize[1], (float)L.height);
         const float sx = mul(add((float)x, add(ox, 0.5f)), dx);

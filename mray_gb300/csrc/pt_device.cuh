@@ -640,12 +640,13 @@ __device__ __forceinline__ float rnd_s(const PtLaunch& L, uint32_t key, uint32_t
     return rnd_zsobol(L, i, bounce, k);
 }
 
-// The bounce's numbers k 0..2 (one Next3D request) or k 4, 5 (one Next2D
-// request) at once; each equals rnd_s of that k.
+// The bounce's numbers k 0..2 (one Next3D request), k 4, 5 (one Next2D
+// request) or, at the camera, k 6, 7 (Next2D) at once; each equals rnd_s of
+// that k.
 __device__ __noinline__ float4 rnd_zsobol_group(const PtLaunch& L, uint32_t i, uint32_t bounce, uint32_t k0)
 {
     const uint32_t b = 3u + 7u * bounce;
-    const uint32_t dim = (k0 == 0u) ? b : b + 4u, size = (k0 == 0u) ? 3u : 2u;
+    const uint32_t dim = (k0 == 6u) ? 0u : (k0 == 0u) ? b : b + 4u, size = (k0 == 0u) ? 3u : 2u;
     const uint32_t pixel = slot_pixel(L, i);
     const ZsGen g = zs_make(pixel % L.width, pixel / L.width, __ldg(L.zsSeeds + pixel), slot_sample(L, i),
                             L.zsMaxSpp, L.zsResBits);
@@ -666,6 +667,14 @@ __device__ __forceinline__ float2 rnd_s45(const PtLaunch& L, uint32_t key, uint3
 {
     if(L.sampler == 0u) return make_float2(rnd(key, bounce, 4), rnd(key, bounce, 5));
     const float4 r = (L.sampler == 3u) ? rnd_pcg32(L, i, bounce, 4u, 2u) : rnd_zsobol_group(L, i, bounce, 4u);
+    return make_float2(r.x, r.y);
+}
+
+// The camera's film-filter numbers, k 6 and 7.
+__device__ __forceinline__ float2 rnd_s67(const PtLaunch& L, uint32_t key, uint32_t i)
+{
+    if(L.sampler == 0u) return make_float2(rnd(key, 0, 6), rnd(key, 0, 7));
+    const float4 r = (L.sampler == 3u) ? rnd_pcg32(L, i, 0u, 6u, 2u) : rnd_zsobol_group(L, i, 0u, 6u);
     return make_float2(r.x, r.y);
 }
 

@@ -97,6 +97,10 @@ void zsobol_tables(uint32_t* out)
     for(int d = 0; d < 4; d++)
         for(int q = 0; q < 24; q++) packed[d] |= (uint64_t)p[q][d] << (2 * q);
     std::memcpy(out + 3 * kZsWidth, packed, sizeof(packed));
+    for(int n = 0; n < kZsNibbles; n++)
+        for(int v = 0; v < 16; v++)
+            for(int j = 0; j < 4; j++)
+                if((v >> j) & 1) out[kZsNibbleWord + 16 * n + v] ^= out[2 * kZsWidth + 4 * n + j];
 }
 
 } // namespace mrg

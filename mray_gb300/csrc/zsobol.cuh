@@ -14,7 +14,11 @@
 namespace mrg {
 
 constexpr int kZsWidth = 52;
-constexpr int kZsTableWords = 3 * kZsWidth + 8;   // matrices, then 4 x uint64 permutations
+constexpr int kZsNibbles = kZsWidth / 4;
+// matrices, 4 x uint64 permutations, then the third matrix by nibbles: word
+// 16 n + v is the sum of its columns 4n + j over the bits j of v
+constexpr int kZsNibbleWord = 3 * kZsWidth + 8;
+constexpr int kZsTableWords = kZsNibbleWord + 16 * kZsNibbles;
 
 // Host: fills the tables (kZsTableWords words) from the Sobol recurrence and
 // the swap enumeration of the permutations of {0, 1, 2, 3}.
@@ -51,23 +55,44 @@ __device__ __forceinline__ uint32_t zs_owen_fast(uint32_t v, uint32_t seed)
     return v;
 }
 
+// The Sobol matrices times the sample index, closed forms where they have one.
+// Dimension 0 is the reversed identity.  Column k of dimension 1 is the
+// polynomial (1 + x)^k, so bit i of the reversed product sums the index bits k
+// with C(k, i) odd, those whose k contains the bits of i (Lucas): a superset
+// sum, five masked shifts (and one fold for index bits 32 and up).  Dimension
+// 2 takes four columns a lookup.  Column by column each took some 6
+// instructions a bit, 22 bits at 333 x 251 x 8 spp.
 __device__ __forceinline__ uint32_t zs_mat_mul(const uint32_t* mat, int d, uint64_t a)
 {
+    if(d == 0) return __brev((uint32_t)a);
+    if(d == 1)
+    {
+        uint32_t y = (uint32_t)a ^ (uint32_t)(a >> 32);
+        y ^= (y >> 1) & 0x55555555u;
+        y ^= (y >> 2) & 0x33333333u;
+        y ^= (y >> 4) & 0x0F0F0F0Fu;
+        y ^= (y >> 8) & 0x00FF00FFu;
+        y ^= y >> 16;
+        return __brev(y);
+    }
     uint32_t r = 0;
-    for(int i = 0; i < kZsWidth && a != 0; i++, a >>= 1)
-        if(a & 1u) r ^= mat[d * kZsWidth + i];
+    for(const uint32_t* t = mat + kZsNibbleWord; a != 0; a >>= 4, t += 16) r ^= t[(uint32_t)a & 15u];
     return r;
 }
 
-__device__ __forceinline__ uint64_t zs_expand2(uint32_t v)
+__device__ __forceinline__ uint32_t zs_expand2_16(uint32_t x)
 {
-    uint64_t x = v;
-    x = (x | (x << 16)) & 0x0000FFFF0000FFFFull;
-    x = (x | (x << 8)) & 0x00FF00FF00FF00FFull;
-    x = (x | (x << 4)) & 0x0F0F0F0F0F0F0F0Full;
-    x = (x | (x << 2)) & 0x3333333333333333ull;
-    x = (x | (x << 1)) & 0x5555555555555555ull;
-    return x;
+    x = (x | (x << 8)) & 0x00FF00FFu;
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    return (x | (x << 1)) & 0x55555555u;
+}
+__device__ __forceinline__ uint64_t zs_morton2(uint32_t x, uint32_t y)
+{
+    const uint32_t lo = zs_expand2_16(x & 0xFFFFu) | (zs_expand2_16(y & 0xFFFFu) << 1);
+    uint32_t hi = 0;
+    if((x | y) >> 16) hi = zs_expand2_16(x >> 16) | (zs_expand2_16(y >> 16) << 1);
+    return (uint64_t)lo | ((uint64_t)hi << 32);
 }
 
 struct ZsGen
@@ -92,22 +117,38 @@ __device__ __forceinline__ ZsGen zs_make(uint32_t px, uint32_t py, uint32_t seed
     }
     g.log2Spp = 31u - __clz(maxSpp);
     g.nDigits = (int32_t)(resMaxBits + (g.log2Spp + 1u) / 2u);
-    g.morton = ((zs_expand2(px) | (zs_expand2(py) << 1)) << g.log2Spp) | local;
+    g.morton = (zs_morton2(px, py) << g.log2Spp) | local;
     g.seed = seed;
     return g;
 }
 
+// zs_mix_bits(v) >> 24, modulo 24: 8 (h mod 3) plus the low three bits, h being
+// the 37 bits above them; 2^16 = 1 mod 3 folds those to 17 bits first.  A
+// 64-bit modulo took three times the instructions.
+__device__ __forceinline__ uint32_t zs_perm_index(uint64_t v)
+{
+    const uint64_t m = zs_mix_bits(v) >> 24;
+    const uint32_t low = (uint32_t)m & 7u;
+    const uint32_t h0 = (uint32_t)(m >> 3), h1 = (uint32_t)(m >> 35);
+    const uint32_t f = (h0 & 0xFFFFu) + (h0 >> 16) + h1;
+    const uint32_t q = __umulhi(f, 0x55555556u);            // f / 3 for f below 2^30
+    return 8u * (f - 3u * q) + low;
+}
+
+// The digits are independent (each hashes the index above it), so they go
+// from the lowest up, the index shifted along instead of by a variable amount.
 __device__ __forceinline__ uint64_t zs_sample_index(const ZsGen& g, const uint64_t* perm, uint32_t dim)
 {
     const uint32_t mixer = 0x55555555u * dim;
-    const bool odd = (g.log2Spp & 1u) != 0u;
-    uint64_t a = 0;
-    for(int32_t q = g.nDigits - 1; q >= (odd ? 1 : 0); q--)
+    const uint32_t odd = g.log2Spp & 1u;
+    uint64_t m = g.morton >> odd, a = 0;
+    uint32_t shift = odd;
+    for(int32_t q = (int32_t)odd; q < g.nDigits; q++, shift += 2u)
     {
-        const uint32_t shift = (uint32_t)(2 * q - (odd ? 1 : 0));
-        const uint32_t digit = (uint32_t)((g.morton >> shift) & 3u);
-        const uint32_t p = (uint32_t)((zs_mix_bits((g.morton >> (shift + 2u)) ^ (uint64_t)mixer) >> 24) % 24u);
-        a |= ((perm[digit] >> (2u * p)) & 3ull) << shift;
+        const uint32_t digit = (uint32_t)m & 3u;
+        m >>= 2;
+        const uint32_t e = (uint32_t)(perm[digit] >> (2u * zs_perm_index(m ^ (uint64_t)mixer))) & 3u;
+        a |= (uint64_t)e << shift;
     }
     if(odd) a |= (g.morton & 1ull) ^ (zs_mix_bits((g.morton >> 1) ^ (uint64_t)mixer) & 1ull);
     return a;
