@@ -232,7 +232,8 @@ typedef struct mrg_pt_params
 {
     uint32_t width, height;      /* film size */
     uint32_t spp;                /* samples per pixel rendered by this call */
-    uint32_t samplesPerPass;     /* paths in flight = width * height * samplesPerPass (0 = auto) */
+    uint32_t samplesPerPass;     /* paths in flight = width * height * samplesPerPass (0 = auto); a
+                                    last pass takes what remains */
     uint32_t rrStart, maxDepth;  /* russianRouletteRange (RR from rrStart, paths end at maxDepth) */
     uint32_t sampleMode;         /* MRG_PT_* */
     uint32_t seed;

@@ -707,11 +707,44 @@ struct PtRun
     mrg::PtSceneTables  T{};
     mrg::TraceScratch   scr{};
     bool                partition = false;
-    uint32_t            spp = 1;       // samples per pass
+    uint32_t            spp = 1;       // samples per pass (the last may have fewer)
     uint32_t            slots = 0;
+
+    uint32_t passes(const mrg_pt_params* p) const { return (p->spp + spp - 1u) / spp; }
+    // the launch of pass k
+    void pass(const mrg_pt_params* p, uint32_t k)
+    {
+        L.samplesPerPass = std::min(spp, p->spp - k * spp);
+        L.slots = p->width * p->height * L.samplesPerPass;
+        L.sampleBase = p->sampleStart + k * spp;
+    }
 };
 
-mrg_status pt_setup(mrg_ctx* c, const mrg_pt_params* p, PtRun& R, cudaStream_t st, const char* who)
+// Samples per pass.  Automatic: as few passes of at most 2^22 paths as it
+// takes, but two (one a pipeline) from 2^19 paths on: a pass of half the size
+// keeps more of its path state in L2, and one pass's casts fill the SMs that
+// the other's last rays leave idle (one -> two: 524k paths
+// 516 -> 504 us, 668k with ZSobol 820 -> 765, 1.05M 863 -> 836, 4.1M 8546 -> 8338;
+// 262k 355 -> 353).  Even passes; a last smaller
+// one where the samples do not divide, unless every pass has to be alike
+// (`even`: each trains the cache or the guiding grid on its paths).
+uint32_t samples_per_pass(const mrg_pt_params* p, bool even)
+{
+    const uint64_t wh = (uint64_t)p->width * p->height;
+    uint32_t spp = p->samplesPerPass;
+    if(!spp && even) spp = std::max<uint32_t>(1, (uint32_t)std::min<uint64_t>(p->spp, (1ull << 22) / wh));
+    if(!spp)
+    {
+        const uint32_t most = std::max<uint32_t>(1, (uint32_t)std::min<uint64_t>(p->spp, (1ull << 22) / wh));
+        uint32_t passes = (p->spp + most - 1u) / most;
+        if(passes == 1u && p->spp >= 2u && wh * p->spp >= (1ull << 19)) passes = 2u;
+        spp = (p->spp + passes - 1u) / passes;
+    }
+    spp = std::min(spp, p->spp);
+    return (even && p->spp % spp != 0) ? 1u : spp;
+}
+
+mrg_status pt_setup(mrg_ctx* c, const mrg_pt_params* p, PtRun& R, cudaStream_t st, const char* who, bool even)
 {
     const std::string w(who);
     if(!c->built) return mrg::set_error(MRG_ERR_NOT_BUILT, w + ": call mrg_build first");
@@ -721,10 +754,7 @@ mrg_status pt_setup(mrg_ctx* c, const mrg_pt_params* p, PtRun& R, cudaStream_t s
         return mrg::set_error(MRG_ERR_INVALID_ARG, w + ": maxDepth must be in [1, 255], sampleMode and "
                                                    "partitionByMaterial in [0, 2]");
     const uint64_t wh = (uint64_t)p->width * p->height;
-    uint32_t spp = p->samplesPerPass ? p->samplesPerPass
-                                     : std::max<uint32_t>(1, (uint32_t)std::min<uint64_t>(p->spp, (1ull << 22) / wh));
-    spp = std::min(spp, p->spp);
-    if(p->spp % spp != 0) spp = 1;
+    const uint32_t spp = samples_per_pass(p, even);
     if(wh * spp > (1ull << 26)) return mrg::set_error(MRG_ERR_LIMIT, w + ": more than 2^26 paths per pass");
     for(uint32_t i = 0; i < c->insts.size(); i++)
         if(i >= c->ptDesc.size() || c->ptDesc[i].kind == 0)
@@ -959,7 +989,7 @@ mrg_status mrg_pt_render(mrg_ctx* c, const mrg_pt_params* p, float* dImage, void
     if(!c || !p || !dImage) return mrg::set_error(MRG_ERR_INVALID_ARG, "mrg_pt_render: null pointer");
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render", false);
     if(s != MRG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     PtLane lanes[2];
@@ -968,13 +998,13 @@ mrg_status mrg_pt_render(mrg_ctx* c, const mrg_pt_params* p, float* dImage, void
     // streams and counters), so one pass's casts fill the SMs the other's
     // leave idle.  Film writes stay in pass order (an event chain); the
     // caller's stream waits for both pipelines at the end.
-    const uint32_t passes = p->spp / R.spp;
+    const uint32_t passes = R.passes(p);
     const bool two = passes >= 2 && pt_two_pipelines();
     if(two && (s = pt_lane1(c, R.slots, st, lanes[0], lanes[1])) != MRG_OK) return s;
     for(uint32_t pass = 0; pass < passes; pass++)
     {
         const PtLane& lane = lanes[two ? (pass & 1u) : 0u];
-        R.L.sampleBase = p->sampleStart + pass * R.spp;
+        R.pass(p, pass);
         PT_TRY(pt_bounces(c, R, lane), "render pass");
         if(two && pass > 0) PT_TRY(cudaStreamWaitEvent(lane.st, c->ptEvFilm, 0), "film order");
         PT_TRY(mrg::pt_film(R.L, *lane.P, reinterpret_cast<float4*>(dImage), lane.st), "film");
@@ -991,7 +1021,7 @@ mrg_status mrg_pt_render_cached(mrg_ctx* c, const mrg_pt_params* p, float* dImag
     constexpr uint32_t kRec = 2;
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render_cached");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render_cached", true);
     if(s != MRG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // buffers: query in / out / list, per-slot training records, batch, counters
@@ -1076,7 +1106,7 @@ mrg_status mrg_pt_adjoint(mrg_ctx* c, const mrg_pt_params* p, uint32_t texId, co
             return mrg::set_error(MRG_ERR_INVALID_ARG, "mrg_pt_adjoint: the parameter texture must feed Lambert albedos");
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_adjoint");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_adjoint", false);
     if(s != MRG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     mrg::PtAdjoint& A = R.L.adj;
@@ -1103,7 +1133,7 @@ mrg_status mrg_pt_adjoint(mrg_ctx* c, const mrg_pt_params* p, uint32_t texId, co
     // atomic adds, so its value does not depend on it
     PtLane lanes[2];
     if((s = pt_lane0(c, st, lanes[0])) != MRG_OK) return s;
-    const uint32_t passes = p->spp / R.spp;
+    const uint32_t passes = R.passes(p);
     const bool two = passes >= 2 && pt_two_pipelines();
     if(two && (s = pt_lane1(c, R.slots, st, lanes[0], lanes[1])) != MRG_OK) return s;
     // Vertex records, or a replay of each pass where they do not fit.  The
@@ -1128,7 +1158,7 @@ mrg_status mrg_pt_adjoint(mrg_ctx* c, const mrg_pt_params* p, uint32_t texId, co
         const uint32_t li = two ? (pass & 1u) : 0u;
         const PtLane& lane = lanes[li];
         float4* radTotal = static_cast<float4*>(li ? c->dPtRadTotal2 : c->dPtRadTotal);
-        R.L.sampleBase = p->sampleStart + pass * R.spp;
+        R.pass(p, pass);
         A.radTotal = radTotal;
         A.mode = replay ? mrg::kAdjOff : mrg::kAdjRecord;
         if(records)
@@ -1146,7 +1176,7 @@ mrg_status mrg_pt_adjoint(mrg_ctx* c, const mrg_pt_params* p, uint32_t texId, co
         if(records) PT_TRY(mrg::pt_adjoint_scatter(R.L, *lane.P, R.T, c->smCount, lane.st), "texture gradient");
         if(replay)
         {
-            PT_TRY(cudaMemcpyAsync(radTotal, lane.P->rad, sizeof(float4) * (size_t)R.slots,
+            PT_TRY(cudaMemcpyAsync(radTotal, lane.P->rad, sizeof(float4) * (size_t)R.L.slots,
                                    cudaMemcpyDeviceToDevice, lane.st), "primal radiance");
             A.mode = mrg::kAdjReplay;
             PT_TRY(pt_bounces(c, R, lane), "replay pass");
@@ -1484,7 +1514,7 @@ mrg_status mrg_pt_render_guided(mrg_ctx* c, const mrg_pt_params* p, float* dImag
         return mrg::set_error(MRG_ERR_INVALID_ARG, "mrg_pt_render_guided: samplers INDEPENDENT and PCG32 only");
     DevGuard g(c->device);
     PtRun R;
-    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render_guided");
+    mrg_status s = pt_setup(c, p, R, static_cast<cudaStream_t>(stream), "mrg_pt_render_guided", true);
     if(s != MRG_OK) return s;
     if((s = guide_paths(c, R.slots)) != MRG_OK) return s;
     if((s = guide_backup_streams(c, p, R.slots, static_cast<cudaStream_t>(stream))) != MRG_OK) return s;
