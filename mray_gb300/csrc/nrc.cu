@@ -108,40 +108,70 @@ __device__ __forceinline__ void sh16(float x, float y, float z, float* o)
     o[15] = 0.59004358992664352f * x * (-xx + 3.0f * yy);
 }
 
-// Writes the 64 input features of sample `s` (valid) into the warp's bf16
-// tile: lane (s, half) encodes levels [8 half, 8 half + 8) and half 0 the
-// direction harmonics, half 1 the normal, albedo, roughness and constants.
-__device__ void encode_sample(const NrcState& S, const float4* in, bool valid, uint32_t half, uint16_t* row)
+// Writes the 64 input features of the warp's 16 samples into their bf16 rows:
+// lanes 2s and 2s + 1 have sample s.
+//
+// The 8 x 16 table reads of a sample bound the query: each brings 4 bytes
+// from a line of its own, and a lookup a cycle is what an SM's L1 does.  So
+// the two lanes read the two x neighbours of a corner together: their entries
+// lie in one 128-byte line in 31 of 32 cases (x and x + 1 hash to indices that
+// differ in low bits only), which makes it one lookup.  Then they trade
+// values, so that each lane has one of two levels whole and sums its corners
+// in the order of one lane per level.  2,073,600 samples, 16 levels of 2^19:
+// 905 -> 598 us.
+__device__ void encode_pair(const NrcState& S, const float4* in, bool valid, uint32_t cx, uint16_t* row)
 {
     const NrcGrid& G = S.grid;
     float4 i0 = make_float4(0, 0, 0, 0), i1 = i0, i2 = i0, i3 = i0;
-    if(valid) { i0 = in[0]; i1 = in[1]; i2 = in[2]; i3 = in[3]; }
+    if(valid)
+    {
+        i0 = in[0];
+        if(cx) { i2 = in[2]; i3 = in[3]; }
+        else i1 = in[1];
+    }
     float ux, uy, uz;
     normalized_pos(G, i0, ux, uy, uz);
     const uint32_t T = 1u << G.log2Table;
 #pragma unroll 2
     for(uint32_t q = 0; q < 8; q++)
     {
-        const uint32_t l = 8u * half + q;
-        float f0 = 0.0f, f1 = 0.0f;
-        if(valid && l < G.levels)
-        {
-            const LevelPos p = level_pos(G, l, ux, uy, uz);
-            const __half2* tab = reinterpret_cast<const __half2*>(S.t16) + (size_t)l * T;
+        uint32_t v[2][4];
+        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
 #pragma unroll
-            for(uint32_t c = 0; c < 8; c++)
+        for(uint32_t t = 0; t < 2; t++)
+        {
+            const uint32_t l = 2u * q + t;
+#pragma unroll
+            for(int j = 0; j < 4; j++) v[t][j] = 0u;
+            if(valid && l < G.levels)
             {
-                const uint32_t cx = c & 1u, cy = (c >> 1) & 1u, cz = (c >> 2) & 1u;
-                const float w = (cx ? p.fx : 1.0f - p.fx) * (cy ? p.fy : 1.0f - p.fy) * (cz ? p.fz : 1.0f - p.fz);
-                const float2 v = __half22float2(__ldg(tab + grid_index(G, l, p.x + cx, p.y + cy, p.z + cz)));
-                f0 += w * v.x;
-                f1 += w * v.y;
+                const LevelPos p = level_pos(G, l, ux, uy, uz);
+                if(t == cx) { fx = p.fx; fy = p.fy; fz = p.fz; }
+                const uint32_t* tab = reinterpret_cast<const uint32_t*>(S.t16) + (size_t)l * T;
+#pragma unroll
+                for(uint32_t j = 0; j < 4; j++)
+                    v[t][j] = __ldg(tab + grid_index(G, l, p.x + cx, p.y + (j & 1u), p.z + (j >> 1)));
             }
         }
-        *reinterpret_cast<uint32_t*>(row + 2 * l) = pack_bf16(f0, f1);
+        float f0 = 0.0f, f1 = 0.0f;
+#pragma unroll
+        for(uint32_t j = 0; j < 4; j++)
+        {
+            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, cx ? v[0][j] : v[1][j], 1);
+            const uint32_t lo = cx ? got : v[0][j], hi = cx ? v[1][j] : got;
+            const float wy = (j & 1u) ? fy : 1.0f - fy, wz = (j >> 1) ? fz : 1.0f - fz;
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&lo));
+            const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+            const float w0 = (1.0f - fx) * wy * wz, w1 = fx * wy * wz;
+            f0 += w0 * a.x;
+            f1 += w0 * a.y;
+            f0 += w1 * c.x;
+            f1 += w1 * c.y;
+        }
+        *reinterpret_cast<uint32_t*>(row + 2u * (2u * q + cx)) = pack_bf16(f0, f1);
     }
     float v[16];
-    if(half == 0u)
+    if(cx == 0u)
     {
         sh16(i1.x, i1.y, i1.z, v);
         if(!valid) for(int k = 0; k < 16; k++) v[k] = 0.0f;
@@ -163,138 +193,120 @@ __device__ void encode_sample(const NrcState& S, const float4* in, bool valid, u
 // Forward: inference (out) or training (stores activations and outputs)
 // ---------------------------------------------------------------------------
 // WARPS warps per CTA share one shared-memory copy of the weights; more warps
-// per CTA keep more hash-grid gathers in flight per SM.
+// per CTA keep more hash-grid gathers in flight per SM.  (32 samples a warp,
+// each weight fragment used twice, measured the same: 597 us against 598, the
+// registers cost as many warps as the reads save.)
 template<bool TRAIN, bool LIST, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 k_nrc_forward(NrcState S, const float4* __restrict__ inputs, const uint32_t* __restrict__ list,
               const uint32_t* nDevice, uint32_t nMax, float4* __restrict__ out)
 {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint16_t* sW = reinterpret_cast<uint16_t*>(smem);                       // (256 + 16) x kPad
+    uint16_t* sW = reinterpret_cast<uint16_t*>(smem);                       // (5 x 64 + 16) x kPad
     uint16_t* sX = sW + (kHiddenRows + kNrcOut) * kPad;                      // WARPS x 16 x kPad
-    float* sO = reinterpret_cast<float*>(sX + WARPS * 16 * kPad);            // WARPS x 16 x 4
-    for(uint32_t i = threadIdx.x; i < (uint32_t)kNrcWeightCount; i += WARPS * 32)
-        sW[(i / kNrcWidth) * kPad + (i % kNrcWidth)] = S.w16[i];
+    // 8 weights a load: a word at a time, staging took a third of a small query
+    for(uint32_t i = threadIdx.x; i < (uint32_t)kNrcWeightCount / 8u; i += WARPS * 32)
+        *reinterpret_cast<uint4*>(sW + (8u * i / kNrcWidth) * kPad + (8u * i % kNrcWidth)) =
+            __ldg(reinterpret_cast<const uint4*>(S.w16) + i);
     __syncthreads();
     const uint32_t n = nDevice ? min(*nDevice, nMax) : nMax;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t g = lane >> 2, t = lane & 3u;
     uint16_t* xw = sX + warp * 16 * kPad;
-    float* ow = sO + warp * 64;
+    float* ow = reinterpret_cast<float*>(xw);                               // outputs, over the input rows
+    // activation `act` of the tile at `base` to memory, as the fragments hold it
+    auto store = [&](const uint32_t (&a)[4][4], uint32_t base, uint32_t act) {
+        uint32_t* A = reinterpret_cast<uint32_t*>(S.acts);
+#pragma unroll
+        for(int kt = 0; kt < 4; kt++)
+        {
+            const uint32_t r0 = base + g, r1 = r0 + 8u;
+            const size_t c = (size_t)act * kNrcWidth + 16 * kt + 2 * t;
+            if(r0 < n)
+            {
+                A[((size_t)r0 * kActs * kNrcWidth + c) / 2] = a[kt][0];
+                A[((size_t)r0 * kActs * kNrcWidth + c + 8) / 2] = a[kt][2];
+            }
+            if(r1 < n)
+            {
+                A[((size_t)r1 * kActs * kNrcWidth + c) / 2] = a[kt][1];
+                A[((size_t)r1 * kActs * kNrcWidth + c + 8) / 2] = a[kt][3];
+            }
+        }
+    };
     for(uint32_t base = (blockIdx.x * WARPS + warp) * 16u; base < n; base += gridDim.x * WARPS * 16u)
     {
         // ---- encode 16 samples ----
         {
-            const uint32_t s = lane & 15u, half = lane >> 4;
-            const uint32_t e = base + s;
+            const uint32_t s = lane >> 1, e = base + s;
             const bool valid = e < n;
             const uint32_t src = valid ? (LIST ? list[e] : e) : 0u;
-            encode_sample(S, inputs + (size_t)src * 4, valid, half, xw + s * kPad);
+            encode_pair(S, inputs + (size_t)src * 4, valid, lane & 1u, xw + s * kPad);
         }
         __syncwarp();
         uint32_t a[4][4];
 #pragma unroll
         for(int kt = 0; kt < 4; kt++)
         {
-            a[kt][0] = lds32(xw + g * kPad + 16 * kt + 2 * t);
-            a[kt][1] = lds32(xw + (g + 8) * kPad + 16 * kt + 2 * t);
-            a[kt][2] = lds32(xw + g * kPad + 16 * kt + 8 + 2 * t);
-            a[kt][3] = lds32(xw + (g + 8) * kPad + 16 * kt + 8 + 2 * t);
+            const uint16_t* r = xw + g * kPad + 16 * kt + 2 * t;
+            a[kt][0] = lds32(r);
+            a[kt][1] = lds32(r + 8 * kPad);
+            a[kt][2] = lds32(r + 8);
+            a[kt][3] = lds32(r + 8 * kPad + 8);
         }
-        if(TRAIN)
-        {
-            // x0 rows as the fragments hold them
-#pragma unroll
-            for(int kt = 0; kt < 4; kt++)
-            {
-                const uint32_t r0 = base + g, r1 = base + g + 8;
-                uint32_t* A = reinterpret_cast<uint32_t*>(S.acts);
-                if(r0 < n)
-                {
-                    A[((size_t)r0 * kActs * kNrcWidth + 16 * kt + 2 * t) / 2] = a[kt][0];
-                    A[((size_t)r0 * kActs * kNrcWidth + 16 * kt + 8 + 2 * t) / 2] = a[kt][2];
-                }
-                if(r1 < n)
-                {
-                    A[((size_t)r1 * kActs * kNrcWidth + 16 * kt + 2 * t) / 2] = a[kt][1];
-                    A[((size_t)r1 * kActs * kNrcWidth + 16 * kt + 8 + 2 * t) / 2] = a[kt][3];
-                }
-            }
-        }
+        if(TRAIN) store(a, base, 0u);
         __syncwarp();
-        // ---- hidden layers ----
+        // ---- hidden layers: two n-tiles give one k-tile of the next layer ----
 #pragma unroll 1
         for(int layer = 0; layer < kNrcHidden; layer++)
         {
             const uint16_t* W = sW + layer * kNrcWidth * kPad;
-            float acc[8][4];
+            uint32_t next[4][4];
 #pragma unroll
-            for(int nt = 0; nt < 8; nt++)
+            for(int kn = 0; kn < 4; kn++)
             {
-                acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
+                float acc[2][4];
 #pragma unroll
-                for(int kt = 0; kt < 4; kt++)
+                for(int h = 0; h < 2; h++)
                 {
-                    const uint16_t* wr = W + (8 * nt + g) * kPad + 16 * kt + 2 * t;
-                    mma_bf16(acc[nt], a[kt], lds32(wr), lds32(wr + 8));
+                    acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.0f;
+#pragma unroll
+                    for(int kt = 0; kt < 4; kt++)
+                    {
+                        const uint16_t* wr = W + (8 * (2 * kn + h) + g) * kPad + 16 * kt + 2 * t;
+                        mma_bf16(acc[h], a[kt], lds32(wr), lds32(wr + 8));
+                    }
                 }
+                next[kn][0] = pack_bf16(fmaxf(acc[0][0], 0.0f), fmaxf(acc[0][1], 0.0f));
+                next[kn][1] = pack_bf16(fmaxf(acc[0][2], 0.0f), fmaxf(acc[0][3], 0.0f));
+                next[kn][2] = pack_bf16(fmaxf(acc[1][0], 0.0f), fmaxf(acc[1][1], 0.0f));
+                next[kn][3] = pack_bf16(fmaxf(acc[1][2], 0.0f), fmaxf(acc[1][3], 0.0f));
             }
 #pragma unroll
             for(int kt = 0; kt < 4; kt++)
-            {
-                a[kt][0] = pack_bf16(fmaxf(acc[2 * kt][0], 0.0f), fmaxf(acc[2 * kt][1], 0.0f));
-                a[kt][1] = pack_bf16(fmaxf(acc[2 * kt][2], 0.0f), fmaxf(acc[2 * kt][3], 0.0f));
-                a[kt][2] = pack_bf16(fmaxf(acc[2 * kt + 1][0], 0.0f), fmaxf(acc[2 * kt + 1][1], 0.0f));
-                a[kt][3] = pack_bf16(fmaxf(acc[2 * kt + 1][2], 0.0f), fmaxf(acc[2 * kt + 1][3], 0.0f));
-            }
-            if(TRAIN)
-            {
-                uint32_t* A = reinterpret_cast<uint32_t*>(S.acts);
-                const size_t off = (size_t)(layer + 1) * kNrcWidth;
 #pragma unroll
-                for(int kt = 0; kt < 4; kt++)
-                {
-                    const uint32_t r0 = base + g, r1 = base + g + 8;
-                    if(r0 < n)
-                    {
-                        A[((size_t)r0 * kActs * kNrcWidth + off + 16 * kt + 2 * t) / 2] = a[kt][0];
-                        A[((size_t)r0 * kActs * kNrcWidth + off + 16 * kt + 8 + 2 * t) / 2] = a[kt][2];
-                    }
-                    if(r1 < n)
-                    {
-                        A[((size_t)r1 * kActs * kNrcWidth + off + 16 * kt + 2 * t) / 2] = a[kt][1];
-                        A[((size_t)r1 * kActs * kNrcWidth + off + 16 * kt + 8 + 2 * t) / 2] = a[kt][3];
-                    }
-                }
-            }
+                for(int q = 0; q < 4; q++) a[kt][q] = next[kt][q];
+            if(TRAIN) store(a, base, (uint32_t)layer + 1u);
         }
-        // ---- output layer (16 rows; the first 3 are RGB) ----
-        float o[2][4];
+        // ---- output layer (16 rows; RGB are columns 0..2 of n-tile 0) ----
+        float o[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
 #pragma unroll
-        for(int nt = 0; nt < 2; nt++)
+        for(int kt = 0; kt < 4; kt++)
         {
-            o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.0f;
-#pragma unroll
-            for(int kt = 0; kt < 4; kt++)
-            {
-                const uint16_t* wr = sW + (kHiddenRows + 8 * nt + g) * kPad + 16 * kt + 2 * t;
-                mma_bf16(o[nt], a[kt], lds32(wr), lds32(wr + 8));
-            }
+            const uint16_t* wr = sW + (kHiddenRows + g) * kPad + 16 * kt + 2 * t;
+            mma_bf16(o, a[kt], lds32(wr), lds32(wr + 8));
         }
-        // columns 0..3 of rows g, g + 8 sit in n-tile 0 with t in {0, 1}
+        // columns 0..3 of rows g, g + 8 sit in the lanes with t in {0, 1}
         if(t < 2u)
         {
-            ow[g * 4 + 2 * t] = o[0][0];
-            ow[g * 4 + 2 * t + 1] = o[0][1];
-            ow[(g + 8) * 4 + 2 * t] = o[0][2];
-            ow[(g + 8) * 4 + 2 * t + 1] = o[0][3];
+            *reinterpret_cast<float2*>(ow + g * 4 + 2 * t) = make_float2(o[0], o[1]);
+            *reinterpret_cast<float2*>(ow + (g + 8) * 4 + 2 * t) = make_float2(o[2], o[3]);
         }
         __syncwarp();
         if(lane < 16u && base + lane < n)
         {
             const uint32_t e = base + lane;
-            const float4 r = make_float4(ow[lane * 4], ow[lane * 4 + 1], ow[lane * 4 + 2], 0.0f);
-            out[LIST ? list[e] : e] = r;
+            out[LIST ? list[e] : e] = make_float4(ow[lane * 4], ow[lane * 4 + 1], ow[lane * 4 + 2], 0.0f);
         }
         __syncwarp();
     }
@@ -313,16 +325,21 @@ k_nrc_backward(NrcState S, const float4* __restrict__ inputs, const float4* __re
     uint16_t* sT = reinterpret_cast<uint16_t*>(smem);                        // 4 x 64 x kPad
     uint16_t* sT4 = sT + kHiddenRows * kPad;                                  // 64 x kPadT4
     float* sG = reinterpret_cast<float*>(sT4 + kNrcWidth * kPadT4);           // WARPS x 16 x 33
-    for(uint32_t i = threadIdx.x; i < (uint32_t)(kHiddenRows * kNrcWidth); i += WARPS * 32)
+    // 8 weights a load, consecutive threads on consecutive rows (their transposed
+    // halves then lie in consecutive places)
+    for(uint32_t i = threadIdx.x; i < (uint32_t)kNrcWeightCount / 8u; i += WARPS * 32)
     {
-        const uint32_t layer = i / (kNrcWidth * kNrcWidth), r = (i / kNrcWidth) % kNrcWidth, c = i % kNrcWidth;
-        // W[layer][out = r][in = c] -> T[layer][in = c][out = r]
-        sT[(layer * kNrcWidth + c) * kPad + r] = S.w16[i];
-    }
-    for(uint32_t i = threadIdx.x; i < (uint32_t)(kNrcOut * kNrcWidth); i += WARPS * 32)
-    {
-        const uint32_t r = i / kNrcWidth, c = i % kNrcWidth;
-        sT4[c * kPadT4 + r] = S.w16[kHiddenRows * kNrcWidth + i];
+        const bool last = i >= (uint32_t)(kHiddenRows * kNrcWidth) / 8u;
+        const uint32_t k = last ? i - (uint32_t)(kHiddenRows * kNrcWidth) / 8u : i % (kNrcWidth * kNrcWidth / 8u);
+        const uint32_t rows = last ? kNrcOut : kNrcWidth, layer = i / (kNrcWidth * kNrcWidth / 8u);
+        const uint32_t r = k % rows, c = 8u * (k / rows);
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(S.w16 + ((size_t)layer * kNrcWidth + r) * kNrcWidth + c));
+        const uint32_t v[4] = { w.x, w.y, w.z, w.w };
+        // W[layer][out = r][in = c ..] -> T[layer][in = c ..][out = r]
+        uint16_t* dst = last ? sT4 + c * kPadT4 + r : sT + (layer * kNrcWidth + c) * kPad + r;
+        const uint32_t pad = last ? kPadT4 : kPad;
+#pragma unroll
+        for(uint32_t q = 0; q < 8u; q++) dst[q * pad] = (uint16_t)(v[q >> 1] >> (16u * (q & 1u)));
     }
     __syncthreads();
     const uint32_t n = nDevice ? min(*nDevice, nMax) : nMax;
@@ -454,7 +471,10 @@ k_nrc_backward(NrcState S, const float4* __restrict__ inputs, const float4* __re
         }
         __syncwarp();
         {
-            const uint32_t s = lane & 15u, half = lane >> 4;
+            // lanes 2s and 2s + 1 have sample s and the two x neighbours of its
+            // corners (one line, mostly); a table entry's two features go
+            // in one reduction
+            const uint32_t s = lane >> 1, cx = lane & 1u;
             const uint32_t e = base + s;
             if(e < n)
             {
@@ -462,21 +482,18 @@ k_nrc_backward(NrcState S, const float4* __restrict__ inputs, const float4* __re
                 float ux, uy, uz;
                 normalized_pos(G, inputs[(size_t)e * 4], ux, uy, uz);
                 const uint32_t T = 1u << G.log2Table;
-                for(uint32_t q = 0; q < 8; q++)
+                for(uint32_t l = 0; l < G.levels; l++)
                 {
-                    const uint32_t l = 8u * half + q;
-                    if(l >= G.levels) break;
                     const float d0 = gw[s * 33 + 2 * l], d1 = gw[s * 33 + 2 * l + 1];
                     const LevelPos p = level_pos(G, l, ux, uy, uz);
-                    float* tab = S.gT + (size_t)l * T * 2;
+                    float2* tab = reinterpret_cast<float2*>(S.gT) + (size_t)l * T;
+                    const float wx = cx ? p.fx : 1.0f - p.fx;
 #pragma unroll
-                    for(uint32_t c = 0; c < 8; c++)
+                    for(uint32_t j = 0; j < 4; j++)
                     {
-                        const uint32_t cx = c & 1u, cy = (c >> 1) & 1u, cz = (c >> 2) & 1u;
-                        const float w = (cx ? p.fx : 1.0f - p.fx) * (cy ? p.fy : 1.0f - p.fy) * (cz ? p.fz : 1.0f - p.fz);
-                        const uint32_t idx = grid_index(G, l, p.x + cx, p.y + cy, p.z + cz);
-                        atomicAdd(tab + 2 * (size_t)idx, w * d0);
-                        atomicAdd(tab + 2 * (size_t)idx + 1, w * d1);
+                        const uint32_t cy = j & 1u, cz = j >> 1;
+                        const float w = wx * (cy ? p.fy : 1.0f - p.fy) * (cz ? p.fz : 1.0f - p.fz);
+                        atomicAdd(tab + grid_index(G, l, p.x + cx, p.y + cy, p.z + cz), make_float2(w * d0, w * d1));
                     }
                 }
             }
@@ -731,7 +748,16 @@ __global__ void k_nrc_wgrad_sum(const float* __restrict__ part, const uint32_t* 
     for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (uint32_t)kNrcWeightCount; i += gridDim.x * blockDim.x)
     {
         float acc = 0.0f;
-        for(uint32_t c = 0; c < used; c++) acc += part[(size_t)c * kNrcWeightCount + i];
+        for(uint32_t c0 = 0; c0 < used; c0 += 40u)           // 40 partials in flight, added in order
+        {
+            float v[40];
+#pragma unroll
+            for(uint32_t c = 0; c < 40u; c++)
+                v[c] = (c0 + c < used) ? part[(size_t)(c0 + c) * kNrcWeightCount + i] : 0.0f;
+#pragma unroll
+            for(uint32_t c = 0; c < 40u; c++)
+                if(c0 + c < used) acc += v[c];
+        }
         gW[i] += acc;
     }
 }
@@ -739,23 +765,54 @@ __global__ void k_nrc_wgrad_sum(const float* __restrict__ part, const uint32_t* 
 // ---------------------------------------------------------------------------
 // Adam (resets the gradient, refreshes the low-precision copy)
 // ---------------------------------------------------------------------------
+// One parameter: moments, step, gradient back to zero; returns the 16-bit copy.
 template<bool HALF>
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, float* __restrict__ gr,
-                       uint16_t* __restrict__ copy, size_t n, float lr, float b1, float b2, float eps, float c1, float c2)
+__device__ __forceinline__ uint16_t adam_one(float& w, float& m, float& v, float& gr, float lr, float b1, float b2,
+                                             float eps, float c1, float c2)
 {
-    for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    const float gi = gr;
+    const float mi = b1 * m + (1.0f - b1) * gi;
+    const float vi = b2 * v + (1.0f - b2) * gi * gi;
+    m = mi;
+    v = vi;
+    const float wi = w - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    w = wi;
+    gr = 0.0f;
+    if(HALF) { __half h = __float2half_rn(wi); return *reinterpret_cast<uint16_t*>(&h); }
+    __nv_bfloat16 h = __float2bfloat16_rn(wi);
+    return *reinterpret_cast<uint16_t*>(&h);
+}
+
+// Four parameters a thread (n is a multiple of 4, the arrays 16-byte aligned):
+// 34 bytes each, 64 of them in flight a thread.  Memory-bound: 16.8M
+// parameters in 84 us (one parameter a thread, 109 us).
+template<bool HALF>
+__global__ void __launch_bounds__(256)
+k_adam(float4* __restrict__ w, float4* __restrict__ m, float4* __restrict__ v, float4* __restrict__ gr,
+       ushort4* __restrict__ copy, size_t n4, float lr, float b1, float b2, float eps, float c1, float c2)
+{
+    for(size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x)
     {
-        const float gi = gr[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = w[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-        w[i] = wi;
-        gr[i] = 0.0f;
-        if(HALF) { __half h = __float2half_rn(wi); copy[i] = *reinterpret_cast<uint16_t*>(&h); }
-        else { __nv_bfloat16 h = __float2bfloat16_rn(wi); copy[i] = *reinterpret_cast<uint16_t*>(&h); }
+        float4 W = w[i], M = m[i], V = v[i], G = gr[i];
+        ushort4 c;
+        c.x = adam_one<HALF>(W.x, M.x, V.x, G.x, lr, b1, b2, eps, c1, c2);
+        c.y = adam_one<HALF>(W.y, M.y, V.y, G.y, lr, b1, b2, eps, c1, c2);
+        c.z = adam_one<HALF>(W.z, M.z, V.z, G.z, lr, b1, b2, eps, c1, c2);
+        c.w = adam_one<HALF>(W.w, M.w, V.w, G.w, lr, b1, b2, eps, c1, c2);
+        w[i] = W; m[i] = M; v[i] = V; gr[i] = G;
+        copy[i] = c;
     }
+}
+
+template<bool HALF>
+void launch_adam(float* w, float* m, float* v, float* gr, uint16_t* copy, size_t n, const NrcState& S, float c1,
+                 float c2, int smCount, cudaStream_t st)
+{
+    const size_t n4 = n / 4;
+    const unsigned grid = (unsigned)std::min<size_t>((n4 + 255) / 256, (size_t)smCount * 8u);
+    k_adam<HALF><<<grid, 256, 0, st>>>(reinterpret_cast<float4*>(w), reinterpret_cast<float4*>(m),
+                                       reinterpret_cast<float4*>(v), reinterpret_cast<float4*>(gr),
+                                       reinterpret_cast<ushort4*>(copy), n4, S.lr, S.beta1, S.beta2, S.eps, c1, c2);
 }
 
 template<bool HALF>
@@ -771,24 +828,29 @@ __global__ void k_copy_params(const float* __restrict__ w, uint16_t* __restrict_
 #ifndef MRG_NRC_QUERY_WARPS
 #define MRG_NRC_QUERY_WARPS 16       // warps per CTA of the inference forward
 #endif
+// Queries of up to this many samples take CTAs of 4 warps, which spread over
+// more SMs and stage their weights sooner: 1,000 samples 10.4 us against 16.6,
+// 20,000 14.6 / 16.6, 80,000 35.0 / 39.1, 160,000 61.6 / 62.7, 400,000 135 / 130,
+// 1,000,000 327 / 305.
+constexpr int kNrcSmallWarps = 4;
+constexpr uint32_t kNrcSmallQuery = 1u << 17;
 constexpr size_t fwd_smem(int warps)
 {
-    return (size_t)(kHiddenRows + kNrcOut) * kPad * 2 + (size_t)warps * 16 * kPad * 2 + (size_t)warps * 64 * 4;
+    return (size_t)(kHiddenRows + kNrcOut) * kPad * 2 + (size_t)warps * 16 * kPad * 2;
 }
 #ifndef MRG_NRC_TRAIN_WARPS
-#define MRG_NRC_TRAIN_WARPS 16       // warps per CTA of the training forward and backward
+#define MRG_NRC_TRAIN_WARPS 4        // warps per CTA of the training forward and backward: a step of 65,536 samples takes
+                                     // 265 us with 4, 261 with 16, 285 with 8; one of 8,000 158, 187, 176
 #endif
 constexpr size_t bwd_smem(int warps)
 {
     return (size_t)kHiddenRows * kPad * 2 + (size_t)kNrcWidth * kPadT4 * 2 + (size_t)warps * 16 * 33 * 4;
 }
 
-template<bool TRAIN, bool LIST>
+template<bool TRAIN, bool LIST, int W>
 cudaError_t launch_forward(const NrcState& S, const float4* in, const uint32_t* list, const uint32_t* nDevice,
                            uint32_t nMax, float4* out, int smCount, cudaStream_t st)
 {
-    // warps per CTA: MRG_NRC_TRAIN_WARPS for training batches, MRG_NRC_QUERY_WARPS for inference
-    constexpr int W = TRAIN ? MRG_NRC_TRAIN_WARPS : MRG_NRC_QUERY_WARPS;
     constexpr size_t smem = fwd_smem(W);
     static int perSMOf[kMaxDevices] = {};          // 0: not configured on that device yet
     int& perSM = perSMOf[launch_device()];
@@ -804,7 +866,7 @@ cudaError_t launch_forward(const NrcState& S, const float4* in, const uint32_t* 
         perSM = b;
     }
     const uint32_t tiles = (nMax + 16 * W - 1) / (16 * W);
-    const uint32_t grid = std::max(1u, std::min(tiles, (uint32_t)smCount * (uint32_t)perSM * 2u));
+    const uint32_t grid = std::max(1u, std::min(tiles, (uint32_t)smCount * (uint32_t)perSM));
     k_nrc_forward<TRAIN, LIST, W><<<grid, W * 32, smem, st>>>(S, in, list, nDevice, nMax, out);
     return cudaGetLastError();
 }
@@ -840,13 +902,17 @@ void nrc_make_grid(NrcGrid& g, uint32_t levels, uint32_t log2Table, uint32_t bas
 cudaError_t nrc_query(const NrcState& S, const float4* inputs, const uint32_t* nDevice, uint32_t nMax,
                       float4* out, int smCount, cudaStream_t st)
 {
-    return launch_forward<false, false>(S, inputs, nullptr, nDevice, nMax, out, smCount, st);
+    return (nMax <= kNrcSmallQuery)
+               ? launch_forward<false, false, kNrcSmallWarps>(S, inputs, nullptr, nDevice, nMax, out, smCount, st)
+               : launch_forward<false, false, MRG_NRC_QUERY_WARPS>(S, inputs, nullptr, nDevice, nMax, out, smCount, st);
 }
 
 cudaError_t nrc_query_list(const NrcState& S, const float4* inputs, const uint32_t* list, const uint32_t* count,
                            uint32_t nMax, float4* out, int smCount, cudaStream_t st)
 {
-    return launch_forward<false, true>(S, inputs, list, count, nMax, out, smCount, st);
+    return (nMax <= kNrcSmallQuery)
+               ? launch_forward<false, true, kNrcSmallWarps>(S, inputs, list, count, nMax, out, smCount, st)
+               : launch_forward<false, true, MRG_NRC_QUERY_WARPS>(S, inputs, list, count, nMax, out, smCount, st);
 }
 
 cudaError_t nrc_train(NrcState& S, const float4* inputs, const float4* targets, const uint32_t* nDevice,
@@ -857,11 +923,9 @@ cudaError_t nrc_train(NrcState& S, const float4* inputs, const float4* targets, 
     S.step += 1;
     const float c1 = 1.0f / (1.0f - std::pow(S.beta1, (float)S.step));
     const float c2 = 1.0f / (1.0f - std::pow(S.beta2, (float)S.step));
-    k_adam<false><<<64, 256, 0, st>>>(S.w32, S.mW, S.vW, S.gW, S.w16, (size_t)kNrcWeightCount, S.lr, S.beta1,
-                                      S.beta2, S.eps, c1, c2);
-    const size_t nt = nrc_table_entries(S.grid) * 2;
-    k_adam<true><<<(unsigned)smCount * 8u, 256, 0, st>>>(S.t32, S.mT, S.vT, S.gT, S.t16, nt, S.lr, S.beta1,
-                                                         S.beta2, S.eps, c1, c2);
+    launch_adam<false>(S.w32, S.mW, S.vW, S.gW, S.w16, (size_t)kNrcWeightCount, S, c1, c2, smCount, st);
+    // levels x 2 << log2Table parameters
+    launch_adam<true>(S.t32, S.mT, S.vT, S.gT, S.t16, nrc_table_entries(S.grid) * 2, S, c1, c2, smCount, st);
     return cudaGetLastError();
 }
 
@@ -885,7 +949,7 @@ cudaError_t nrc_gradients(NrcState& S, const float4* inputs, const float4* targe
     }
     cudaError_t e = cudaMemsetAsync(S.loss, 0, sizeof(float), st);
     // the forward stores the activations and the outputs of the batch
-    if(e == cudaSuccess) e = launch_forward<true, false>(S, inputs, nullptr, nDevice, nMax, S.y, smCount, st);
+    if(e == cudaSuccess) e = launch_forward<true, false, MRG_NRC_TRAIN_WARPS>(S, inputs, nullptr, nDevice, nMax, S.y, smCount, st);
     const uint32_t tiles = (nMax + 16 * W - 1) / (16 * W);
     const uint32_t grid = std::max(1u, std::min(tiles, (uint32_t)smCount * (uint32_t)perSM * 2u));
     if(e == cudaSuccess)
