@@ -110,7 +110,7 @@ enum TraceErrorBits : uint32_t
 };
 
 // nDevice (optional): device word holding the ray count, read by the kernel
-// (device-driven wavefronts); when given, n is ignored.
+// (device-driven wavefronts); when given, n is an upper bound (0: unknown).
 // Listed ray i against instance instIds[i] only (CastLocalRays).
 cudaError_t launch_local(const TraceScene& sc, const TraceScratch& scr, void* rays, const uint32_t* rayIdx,
                          const uint32_t* instIds, uint32_t n, void* hits, void* meta, int smCount, cudaStream_t st);
@@ -124,7 +124,7 @@ cudaError_t launch_visibility(const TraceScene& sc, const TraceScratch& scr, uin
 // that reaches its light adds its radiance shadowRad[i] to rad[i]
 // (KCAccumulateShadowRaysPT) where the cast ends.
 cudaError_t launch_shadow(const TraceScene& sc, const TraceScratch& scr, const void* rays, const uint32_t* rayIdx,
-                          const uint32_t* nDevice, const float4* shadowRad, float4* rad, int smCount,
+                          uint32_t n, const uint32_t* nDevice, const float4* shadowRad, float4* rad, int smCount,
                           cudaStream_t st);
 // Loads the closest-hit traversal kernel on the current device (a function
 // attribute query forces a lazily loaded module in).

@@ -879,7 +879,7 @@ cudaError_t pt_bounces(mrg_ctx* c, PtRun& R, const PtLane& lane)
     for(uint32_t depth = 0; depth < loops && e == cudaSuccess; depth++)
     {
         const PtBounce B(P, R.scr, depth, R.partition);
-        e = mrg::launch_closest(c->scene, B.closest, P.rays, B.alive, 0, P.hits, P.meta, c->smCount, st,
+        e = mrg::launch_closest(c->scene, B.closest, P.rays, B.alive, L.slots, P.hits, P.meta, c->smCount, st,
                                 B.ctr + mrg::kCtrAlive);
         if(e == cudaSuccess && R.partition)
             e = mrg::pt_group(L, P, R.T.surfaces, R.T.nSurfaces, B.alive, B.ctr, st);
@@ -890,14 +890,14 @@ cudaError_t pt_bounces(mrg_ctx* c, PtRun& R, const PtLane& lane)
         if(e == cudaSuccess && overlap) e = cudaStreamWaitEvent(side, lane.evShaded, 0);
         if(e == cudaSuccess && emission)
         {
-            e = mrg::launch_visibility(c->scene, B.shadow, P.visBits, P.shadowRays, P.shadowList, 0, c->smCount, side,
+            e = mrg::launch_visibility(c->scene, B.shadow, P.visBits, P.shadowRays, P.shadowList, L.slots, c->smCount, side,
                                        B.ctr + mrg::kCtrShadow);
             if(e == cudaSuccess)
                 e = mrg::pt_resolve_emission(L, P, R.T.lights, B.ctr + mrg::kCtrShadow, c->smCount, side);
         }
         else if(e == cudaSuccess)
-            e = mrg::launch_shadow(c->scene, B.shadow, P.shadowRays, P.shadowList, B.ctr + mrg::kCtrShadow,
-                                   P.shadowRad, P.rad, c->smCount, side);
+            e = mrg::launch_shadow(c->scene, B.shadow, P.shadowRays, P.shadowList, L.slots,
+                                   B.ctr + mrg::kCtrShadow, P.shadowRad, P.rad, c->smCount, side);
         if(e == cudaSuccess && overlap) e = cudaEventRecord(lane.evResolved, side);
     }
     if(e == cudaSuccess && overlap) e = cudaStreamWaitEvent(st, lane.evResolved, 0);
@@ -1347,7 +1347,7 @@ cudaError_t guided_bounces(mrg_ctx* c, PtRun& R, const PtLane& lane)
     {
         const PtBounce B(P, R.scr, depth, R.partition);
         const uint32_t* aliveCount = B.ctr + mrg::kCtrAlive;
-        e = mrg::launch_closest(c->scene, B.closest, P.rays, B.alive, 0, P.hits, P.meta, c->smCount, st, aliveCount);
+        e = mrg::launch_closest(c->scene, B.closest, P.rays, B.alive, L.slots, P.hits, P.meta, c->smCount, st, aliveCount);
         if(e == cudaSuccess && R.partition)
             e = mrg::pt_group(L, P, R.T.surfaces, R.T.nSurfaces, B.alive, B.ctr, st);
         if(e == cudaSuccess && overlap && depth > 0) e = cudaStreamWaitEvent(st, lane.evResolved, 0);
@@ -1358,7 +1358,7 @@ cudaError_t guided_bounces(mrg_ctx* c, PtRun& R, const PtLane& lane)
         if(e == cudaSuccess && overlap) e = cudaEventRecord(lane.evShaded, st);
         if(e == cudaSuccess && overlap) e = cudaStreamWaitEvent(side, lane.evShaded, 0);
         if(e == cudaSuccess)
-            e = mrg::launch_visibility(c->scene, B.shadow, P.visBits, P.shadowRays, P.shadowList, 0, c->smCount, side,
+            e = mrg::launch_visibility(c->scene, B.shadow, P.visBits, P.shadowRays, P.shadowList, L.slots, c->smCount, side,
                                        B.ctr + mrg::kCtrShadow);
         if(e == cudaSuccess) e = mrg::guide_resolve(P, Q, B.ctr + mrg::kCtrShadow, c->smCount, side);
         if(e == cudaSuccess) e = mrg::guide_apply(G, Q, c->smCount, side);

@@ -56,6 +56,7 @@ constexpr uint32_t kStepCap = 1u << 24;
 constexpr int kRefillMin = MRG_TRACE_REFILL;
 constexpr int kStepBudget = MRG_TRACE_STEP_BUDGET;
 constexpr int kPostponeLanes = MRG_TRACE_POSTPONE;
+constexpr uint32_t kSpread = 2;
 
 struct LevelRay
 {
@@ -212,7 +213,11 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* __restrict__ 
 // WT: the watertight triangle test on records that hold the three vertices.
 // ADD (with ANY): an unoccluded ray adds its radiance to its path (hits the
 // path radiance, meta the rays' radiance) instead of setting a visibility bit.
-template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false>
+// FEW: the cast has fewer rays than the grid has lanes.  A cast lasts as long
+// as its slowest warp, and a warp's pass costs its divergent lanes' paths one
+// after another, so the rays are spread: a warp keeps at most its share of
+// them (kSpread times it, at least one) in its first lanes and the rest idle.
+template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false, bool FEW = false>
 __global__ void __launch_bounds__(kTraceTPB, MRG_TRACE_MIN_BLOCKS)
 k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
         const uint32_t* __restrict__ rayIdx, uint32_t nHost, const uint32_t* __restrict__ nDevice,
@@ -263,11 +268,20 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
     float instTBefore = 0.0f;
     bool warpDone = false;
 
+    uint32_t share = 32u;
+    if(FEW)
+    {
+        const uint32_t warps = gridDim.x * (kTraceTPB / 32);
+        share = min(32u, max(1u, (n * kSpread + warps - 1u) / warps));
+    }
+    const uint32_t ours = 0xFFFFFFFFu >> (32u - share);
+    const int refillMin = FEW ? min(kRefillMin, (int)share) : kRefillMin;
+
     for(;;)
     {
         // ---- refill idle lanes (warp-uniform decision) ------------------------
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !live);
-        if(!warpDone && __popc(idle) >= kRefillMin)
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !live) & (FEW ? ours : 0xFFFFFFFFu);
+        if(!warpDone && __popc(idle) >= refillMin)
         {
             const uint32_t cnt = __popc(idle);
             const int leader = __ffs(idle) - 1;
@@ -275,7 +289,7 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
             if((int)lane == leader) base = atomicAdd(scr.workCounter, cnt);
             base = __shfl_sync(0xFFFFFFFFu, base, leader);
             if(base + cnt >= n) warpDone = true;
-            if(!live)
+            if(FEW ? ((idle >> lane) & 1u) != 0u : !live)
             {
                 const uint32_t i = base + __popc(idle & laneLt);
                 if(i < n)
@@ -529,7 +543,7 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
     }
 }
 
-template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false>
+template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false, bool FEW = false>
 int blocks_for(int smCount)
 {
     static int perSMOf[kMaxDevices] = {};          // 0: not queried on that device yet
@@ -537,8 +551,8 @@ int blocks_for(int smCount)
     if(perSM == 0)
     {
         int b = 0;
-        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace<ANY, STATS, LOCAL, WT, ADD>, kTraceTPB, 0) != cudaSuccess ||
-           b < 1)
+        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace<ANY, STATS, LOCAL, WT, ADD, FEW>, kTraceTPB, 0) !=
+               cudaSuccess || b < 1)
             b = 4;
         perSM = b;
     }
@@ -548,6 +562,33 @@ int blocks_for(int smCount)
 cudaError_t clear_counter(const TraceScratch& scr, cudaStream_t st)
 {
     return scr.cleared ? cudaSuccess : cudaMemsetAsync(scr.workCounter, 0, sizeof(uint32_t), st);
+}
+
+// A cast of n rays (with a device-side count: of at most n, 0: unknown).  FEW
+// while a warp's share stays below 32, some 68,000 rays: beyond that it only
+// costs registers (3.95M rays: 1.5%).  Closest hit on 27 x 82k triangles,
+// 1,000 / 4,000 / 16,000 / 64,000 rays: 76 / 89 / 112 / 123 us filling the
+// warps, 56 / 70 / 90 / 124 spread; any hit 87 / 94 / 108 / 125 and 56 / 66 /
+// 93 / 122.  (Twice the even share: 1x and 4x gave 92 and 100 us at 16,000.
+// A kernel of eight lanes a ray, a child each, took 62 / 75 / 98 / 173 with
+// four rays a warp, 57 / 72 / 122 with one: the chain of node loads remains.)
+template<bool ANY, bool WT, bool ADD = false>
+cudaError_t launch_cast(const TraceScene& sc, const TraceScratch& scr, const void* rays, const uint32_t* rayIdx,
+                        uint32_t n, const uint32_t* nDevice, void* hits, void* meta, uint32_t* visBits, int smCount,
+                        cudaStream_t st)
+{
+    cudaError_t e = clear_counter(scr, st);
+    if(e != cudaSuccess) return e;
+    float4* r = const_cast<float4*>(static_cast<const float4*>(rays));
+    uint4* h = static_cast<uint4*>(hits);
+    float2* m = static_cast<float2*>(meta);
+    const int few = blocks_for<ANY, false, false, WT, ADD, true>(smCount);
+    if(n != 0u && n <= (uint32_t)few * kTraceTPB / kSpread)
+        k_trace<ANY, false, false, WT, ADD, true><<<few, kTraceTPB, 0, st>>>(sc, scr, r, rayIdx, n, nDevice, h, m, visBits);
+    else
+        k_trace<ANY, false, false, WT, ADD><<<blocks_for<ANY, false, false, WT, ADD>(smCount), kTraceTPB, 0, st>>>(
+            sc, scr, r, rayIdx, n, nDevice, h, m, visBits);
+    return cudaGetLastError();
 }
 
 } // namespace
@@ -563,17 +604,8 @@ cudaError_t launch_closest(const TraceScene& sc, const TraceScratch& scr, void* 
                            int smCount, cudaStream_t st, const uint32_t* nDevice)
 {
     if(n == 0 && nDevice == nullptr) return cudaSuccess;
-    cudaError_t e = clear_counter(scr, st);
-    if(e != cudaSuccess) return e;
-    if(sc.watertight)
-        k_trace<false, false, false, true><<<blocks_for<false, false, false, true>(smCount), kTraceTPB, 0, st>>>(
-            sc, scr, static_cast<float4*>(rays), rayIdx, n, nDevice, static_cast<uint4*>(hits),
-            static_cast<float2*>(meta), nullptr);
-    else
-        k_trace<false, false><<<blocks_for<false, false>(smCount), kTraceTPB, 0, st>>>(
-            sc, scr, static_cast<float4*>(rays), rayIdx, n, nDevice, static_cast<uint4*>(hits),
-            static_cast<float2*>(meta), nullptr);
-    return cudaGetLastError();
+    return sc.watertight ? launch_cast<false, true>(sc, scr, rays, rayIdx, n, nDevice, hits, meta, nullptr, smCount, st)
+                         : launch_cast<false, false>(sc, scr, rays, rayIdx, n, nDevice, hits, meta, nullptr, smCount, st);
 }
 
 cudaError_t launch_local(const TraceScene& sc, const TraceScratch& scr, void* rays, const uint32_t* rayIdx,
@@ -598,35 +630,17 @@ cudaError_t launch_visibility(const TraceScene& sc, const TraceScratch& scr, uin
                               int smCount, cudaStream_t st, const uint32_t* nDevice)
 {
     if(n == 0 && nDevice == nullptr) return cudaSuccess;
-    cudaError_t e = clear_counter(scr, st);
-    if(e != cudaSuccess) return e;
-    if(sc.watertight)
-        k_trace<true, false, false, true><<<blocks_for<true, false, false, true>(smCount), kTraceTPB, 0, st>>>(
-            sc, scr, const_cast<float4*>(static_cast<const float4*>(rays)), rayIdx, n, nDevice, nullptr,
-            nullptr, visBits);
-    else
-        k_trace<true, false><<<blocks_for<true, false>(smCount), kTraceTPB, 0, st>>>(
-            sc, scr, const_cast<float4*>(static_cast<const float4*>(rays)), rayIdx, n, nDevice, nullptr,
-            nullptr, visBits);
-    return cudaGetLastError();
+    return sc.watertight ? launch_cast<true, true>(sc, scr, rays, rayIdx, n, nDevice, nullptr, nullptr, visBits, smCount, st)
+                         : launch_cast<true, false>(sc, scr, rays, rayIdx, n, nDevice, nullptr, nullptr, visBits, smCount, st);
 }
 
 cudaError_t launch_shadow(const TraceScene& sc, const TraceScratch& scr, const void* rays, const uint32_t* rayIdx,
-                          const uint32_t* nDevice, const float4* shadowRad, float4* rad, int smCount,
+                          uint32_t n, const uint32_t* nDevice, const float4* shadowRad, float4* rad, int smCount,
                           cudaStream_t st)
 {
-    cudaError_t e = clear_counter(scr, st);
-    if(e != cudaSuccess) return e;
-    float4* r = const_cast<float4*>(static_cast<const float4*>(rays));
-    uint4* out = reinterpret_cast<uint4*>(rad);
-    float2* add = reinterpret_cast<float2*>(const_cast<float4*>(shadowRad));
-    if(sc.watertight)
-        k_trace<true, false, false, true, true><<<blocks_for<true, false, false, true, true>(smCount), kTraceTPB, 0,
-                                                  st>>>(sc, scr, r, rayIdx, 0, nDevice, out, add, nullptr);
-    else
-        k_trace<true, false, false, false, true><<<blocks_for<true, false, false, false, true>(smCount), kTraceTPB, 0,
-                                                   st>>>(sc, scr, r, rayIdx, 0, nDevice, out, add, nullptr);
-    return cudaGetLastError();
+    void* add = const_cast<float4*>(shadowRad);
+    return sc.watertight ? launch_cast<true, true, true>(sc, scr, rays, rayIdx, n, nDevice, rad, add, nullptr, smCount, st)
+                         : launch_cast<true, false, true>(sc, scr, rays, rayIdx, n, nDevice, rad, add, nullptr, smCount, st);
 }
 
 cudaError_t launch_closest_stats(const TraceScene& sc, const TraceScratch& scr, const void* rays,
