@@ -7,7 +7,7 @@
 //      in double, which is slow on this part and changes only the tree shape)
 //   3. radix sort of (code, leaf)            (CUB DeviceRadixSort, build only)
 //   4. Karras 2012 binary radix tree         (k_karras)
-//   5. bottom-up boxes + leaf counts         (k_bottom_up; fence + atomic)
+//   5. bottom-up boxes and SAH costs         (k_bottom_up; fence + atomic)
 //   6. top-down collapse to 8-wide nodes     (k_collapse, one launch per level)
 //      with 8-bit quantised child boxes, up to `maxLeaf` primitives per leaf
 //      child, children placed in slots by direction so that traversal visits
@@ -180,27 +180,30 @@ __global__ void k_morton(const float* __restrict__ cent, const uint32_t* __restr
 }
 
 // Batched BLAS build, leaves of every mesh: box, centroid, per-mesh centroid
-// bounds.  A block whose leaves all belong to one mesh reduces in shared
-// memory first; a block that straddles meshes uses per-leaf atomics.
-__global__ void k_leaf_boxes_multi(const MeshSeg* __restrict__ segs, const uint32_t* __restrict__ firsts,
-                                   uint32_t nMesh, uint32_t n, BoxF* __restrict__ boxes, float* __restrict__ cent,
-                                   uint32_t* __restrict__ cbounds, uint32_t* __restrict__ leafMesh)
+// bounds.  Lanes of one mesh reduce in registers first; a block whose leaves
+// all belong to one mesh then reduces in shared memory, others leave an atomic
+// a bound, mesh and warp.  509 meshes of 320 triangles: 33 us with an atomic a
+// lane and bound, 6 now.
+__global__ void __launch_bounds__(kTPB)
+k_leaf_boxes_multi(const MeshSeg* __restrict__ segs, const uint32_t* __restrict__ firsts, uint32_t nMesh, uint32_t n,
+                   BoxF* __restrict__ boxes, float* __restrict__ cent, uint32_t* __restrict__ cbounds,
+                   uint32_t* __restrict__ leafMesh)
 {
     __shared__ uint32_t sb[6];
-    __shared__ uint32_t blockMesh;
+    __shared__ uint32_t ends[2];                  // mesh of the block's first and last leaf
     const uint32_t b0 = blockIdx.x * blockDim.x;
-    const uint32_t b1 = min(n, b0 + blockDim.x) - 1u;
     if(threadIdx.x < 6) sb[threadIdx.x] = (threadIdx.x < 3) ? 0xFFFFFFFFu : 0u;
-    if(threadIdx.x == 0)
-    {
-        const uint32_t m0 = mesh_of(firsts, nMesh, b0), m1 = mesh_of(firsts, nMesh, b1);
-        blockMesh = (m0 == m1) ? m0 : 0xFFFFFFFFu;
-    }
+    if((threadIdx.x & 31u) == 0u && threadIdx.x < 64u)
+        ends[threadIdx.x >> 5] = mesh_of(firsts, nMesh, threadIdx.x ? min(n, b0 + blockDim.x) - 1u : b0);
     __syncthreads();
+    const bool single = ends[0] == ends[1];
     const uint32_t i = b0 + threadIdx.x;
-    if(i < n)
+    const bool in = i < n;
+    uint32_t m = ends[0];
+    uint32_t lo[3] = { 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu }, hi[3] = { 0u, 0u, 0u };
+    if(in)
     {
-        const uint32_t m = mesh_of(firsts, nMesh, i);
+        while(m < ends[1] && firsts[m + 1] <= i) m++;
         const MeshSeg& sg = segs[m];
         const uint32_t t = i - sg.first;
         const uint32_t a = sg.idx[3 * t], b = sg.idx[3 * t + 1], c = sg.idx[3 * t + 2];
@@ -212,26 +215,24 @@ __global__ void k_leaf_boxes_multi(const MeshSeg* __restrict__ segs, const uint3
             bx.mx[k] = fmaxf(va, fmaxf(vb, vc));
             const float cc = 0.5f * (bx.mn[k] + bx.mx[k]);
             cent[3 * i + k] = cc;
-            if(blockMesh != 0xFFFFFFFFu)
-            {
-                atomicMin(&sb[k], f2ord(cc));
-                atomicMax(&sb[3 + k], f2ord(cc));
-            }
-            else
-            {
-                atomicMin(&cbounds[6 * m + k], f2ord(cc));
-                atomicMax(&cbounds[6 * m + 3 + k], f2ord(cc));
-            }
+            lo[k] = hi[k] = f2ord(cc);
         }
         boxes[i] = bx;
         leafMesh[i] = m;
     }
-    __syncthreads();
-    if(blockMesh != 0xFFFFFFFFu)
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, in ? m : 0xFFFFFFFFu);
+    const bool leader = in && (threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1u;
+    uint32_t* const bounds = single ? sb : cbounds + 6 * (size_t)m;
+#pragma unroll
+    for(int k = 0; k < 3; k++)
     {
-        if(threadIdx.x < 3) atomicMin(&cbounds[6 * blockMesh + threadIdx.x], sb[threadIdx.x]);
-        else if(threadIdx.x < 6) atomicMax(&cbounds[6 * blockMesh + threadIdx.x], sb[threadIdx.x]);
+        const uint32_t l = __reduce_min_sync(peers, lo[k]), h = __reduce_max_sync(peers, hi[k]);
+        if(leader) { atomicMin(&bounds[k], l); atomicMax(&bounds[3 + k], h); }
     }
+    if(!single) return;
+    __syncthreads();
+    if(threadIdx.x < 3) atomicMin(&cbounds[6 * (size_t)m + threadIdx.x], sb[threadIdx.x]);
+    else if(threadIdx.x < 6) atomicMax(&cbounds[6 * (size_t)m + threadIdx.x], sb[threadIdx.x]);
 }
 
 // Keys of a batched build: mesh id above a Morton code of `bits` bits per
@@ -288,12 +289,13 @@ __device__ __forceinline__ int k_delta(const uint64_t* __restrict__ c, int n, in
 }
 
 // Karras 2012, "Maximizing parallelism in the construction of BVHs".  In a
-// batched build (firsts != null) the mesh id heads every key, so each mesh's
-// leaves form one subtree; the node whose range is exactly a mesh's leaves
-// is recorded as that mesh's root.
+// batched build (firsts != null) the mesh id heads every key, above its low
+// `meshShift` bits, so each mesh's leaves form one subtree; the node whose
+// range is exactly a mesh's leaves is recorded as that mesh's root.  Nodes that
+// span meshes belong to no tree: they stay nobody's parent.
 __global__ void k_karras(const uint64_t* __restrict__ codes, int n, BinNode* __restrict__ nodes,
                          uint32_t* __restrict__ leafParent, const uint32_t* __restrict__ firsts,
-                         uint32_t nMesh, uint32_t* __restrict__ meshRoot)
+                         uint32_t meshShift, uint32_t* __restrict__ meshRoot)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n - 1) return;
@@ -316,65 +318,18 @@ __global__ void k_karras(const uint64_t* __restrict__ codes, int n, BinNode* __r
     int gamma = i + s * d + min(d, 0);
     int lo = min(i, j), hi = max(i, j);
     BinNode& me = nodes[i];
-    if(lo == gamma) { me.left = kLeafBit | (uint32_t)gamma; leafParent[gamma] = (uint32_t)i; }
-    else            { me.left = (uint32_t)gamma; nodes[gamma].parent = (uint32_t)i; }
-    if(hi == gamma + 1) { me.right = kLeafBit | (uint32_t)(gamma + 1); leafParent[gamma + 1] = (uint32_t)i; }
-    else                { me.right = (uint32_t)(gamma + 1); nodes[gamma + 1].parent = (uint32_t)i; }
+    const bool within = !firsts || ((codes[i] ^ codes[j]) >> meshShift) == 0u;
+    const uint32_t up = within ? (uint32_t)i : kNoParent;
+    me.leafCount = (uint32_t)(hi - lo) + 1u;
+    if(lo == gamma) { me.left = kLeafBit | (uint32_t)gamma; leafParent[gamma] = up; }
+    else            { me.left = (uint32_t)gamma; nodes[gamma].parent = up; }
+    if(hi == gamma + 1) { me.right = kLeafBit | (uint32_t)(gamma + 1); leafParent[gamma + 1] = up; }
+    else                { me.right = (uint32_t)(gamma + 1); nodes[gamma + 1].parent = up; }
     if(i == 0) me.parent = kNoParent;
-    if(firsts)
+    if(firsts && within)
     {
-        const uint32_t m = mesh_of(firsts, nMesh, (uint32_t)lo);
+        const uint32_t m = (uint32_t)(codes[i] >> meshShift);
         if((uint32_t)lo == firsts[m] && (uint32_t)hi + 1u == firsts[m + 1]) meshRoot[m] = (uint32_t)i;
-    }
-}
-
-// Bottom-up boxes and leaf counts.  The second thread to reach a node merges
-// its children.  Writers fence before the counter atomic; readers of another
-// thread's node box load through L2 (__ldcg) since L1 is not coherent.
-__global__ void k_bottom_up(const uint32_t* __restrict__ leafParent, const uint32_t* __restrict__ sortedIds,
-                            const BoxF* __restrict__ leafBoxes, BinNode* nodes, BoxF* nodeBoxes,
-                            uint32_t* counters, int n, uint32_t* errorFlag)
-{
-    int li = blockIdx.x * blockDim.x + threadIdx.x;
-    if(li >= n) return;
-    const uint32_t nInt = (uint32_t)(n - 1);
-    uint32_t p = leafParent[li];
-    for(int guard = 0; p != kNoParent; guard++)
-    {
-        if(p >= nInt || guard > n) { atomicOr(errorFlag, 1u); return; }
-        uint32_t old = atomicAdd(&counters[p], 1u);
-        if(old == 0) return;
-        __threadfence();
-        uint32_t ch[2] = { __ldcg(&nodes[p].left), __ldcg(&nodes[p].right) };
-        for(int c = 0; c < 2; c++)
-        {
-            const bool leaf = (ch[c] & kLeafBit) != 0u;
-            const uint32_t ix = ch[c] & ~kLeafBit;
-            if((leaf && ix >= (uint32_t)n) || (!leaf && ix >= nInt)) { atomicOr(errorFlag, 1u); return; }
-        }
-        BoxF b;
-        uint32_t cnt = 0;
-        for(int k = 0; k < 3; k++) { b.mn[k] = FLT_MAX; b.mx[k] = -FLT_MAX; }
-        for(int c = 0; c < 2; c++)
-        {
-            BoxF cb;
-            if(ch[c] & kLeafBit)
-            {
-                cb = leafBoxes[sortedIds[ch[c] & ~kLeafBit]];
-                cnt += 1;
-            }
-            else
-            {
-                const float* src = reinterpret_cast<const float*>(&nodeBoxes[ch[c]]);
-                for(int k = 0; k < 3; k++) { cb.mn[k] = __ldcg(src + k); cb.mx[k] = __ldcg(src + 3 + k); }
-                cnt += __ldcg(&nodes[ch[c]].leafCount);
-            }
-            for(int k = 0; k < 3; k++) { b.mn[k] = fminf(b.mn[k], cb.mn[k]); b.mx[k] = fmaxf(b.mx[k], cb.mx[k]); }
-        }
-        nodeBoxes[p] = b;
-        nodes[p].leafCount = cnt;
-        __threadfence();
-        p = __ldcg(&nodes[p].parent);
     }
 }
 
@@ -392,7 +347,7 @@ __global__ void k_bottom_up(const uint32_t* __restrict__ leafParent, const uint3
 // wide node's root by its recorded choices instead of greedily opening the
 // largest child.
 // ---------------------------------------------------------------------------
-struct WideCost
+struct __align__(16) WideCost
 {
     float   c[8];          // C(n, i), i = 1..8
     uint8_t split[8];      // for i >= 2: 0 = C(n, i - 1), else k of D(n, i)
@@ -400,82 +355,130 @@ struct WideCost
     uint32_t asLeaf;       // 1: n is a leaf child (it fits one and that is cheaper)
 };
 
-__device__ __forceinline__ float ref_cost(const WideCost* costs, const BoxF* __restrict__ leafBoxes,
-                                          const uint32_t* __restrict__ sortedIds, uint32_t ref, int i, float cPrim)
+__device__ __forceinline__ float box_cost_area(const BoxF& b)
 {
-    if(ref & kLeafBit)
-    {
-        const BoxF b = leafBoxes[sortedIds[ref & ~kLeafBit]];
-        const float dx = b.mx[0] - b.mn[0], dy = b.mx[1] - b.mn[1], dz = b.mx[2] - b.mn[2];
-        return cPrim * (dx * dy + dy * dz + dz * dx);
-    }
-    return __ldcg(&costs[ref].c[i - 1]);
+    const float dx = b.mx[0] - b.mn[0], dy = b.mx[1] - b.mn[1], dz = b.mx[2] - b.mn[2];
+    return dx * dy + dy * dz + dz * dx;
 }
 
-__global__ void k_wide_cost(const uint32_t* __restrict__ leafParent, const uint32_t* __restrict__ sortedIds,
-                            const BoxF* __restrict__ leafBoxes, const BinNode* __restrict__ nodes,
-                            const BoxF* __restrict__ nodeBoxes, WideCost* costs, uint32_t* counters, int n,
-                            const uint32_t* __restrict__ firsts, const MeshSeg* __restrict__ segs, uint32_t nMesh,
-                            uint32_t maxLeaf, float cNode, float cPrim, uint32_t* errorFlag)
+// Bottom-up boxes and, SAH, costs.  A thread climbs from its leaf; the second
+// to reach a node merges the sibling's data with what it holds itself, and
+// goes on.  Writers fence before the counter atomic; the sibling's data are
+// loaded through L2 (__ldcg) since L1 is not coherent.  Bound by the chain of
+// an atomic, a load and a fence a level: the node comes with the atomic, and
+// boxes and costs go up together, no further than a mesh's root.  Two climbs,
+// over the meshes' common top as well, took 128 us for 509 meshes of 320
+// triangles and 598 for one of 1.3M; this one 34 and 277.
+template<bool SAH>
+__global__ void __launch_bounds__(kTPB)
+k_bottom_up(const uint32_t* __restrict__ leafParent, const uint32_t* __restrict__ sortedIds,
+            const BoxF* __restrict__ leafBoxes, const BinNode* __restrict__ nodes, BoxF* nodeBoxes, WideCost* costs,
+            uint32_t* counters, int n, const uint64_t* __restrict__ codes, uint32_t meshShift,
+            const MeshSeg* __restrict__ segs, uint32_t maxLeaf, float cNode, float cPrim, uint32_t* errorFlag)
 {
     const int li = blockIdx.x * blockDim.x + threadIdx.x;
     if(li >= n) return;
     const uint32_t nInt = (uint32_t)(n - 1);
-    const uint32_t ml = segs ? segs[mesh_of(firsts, nMesh, (uint32_t)li)].maxLeaf : maxLeaf;
     uint32_t p = leafParent[li];
+    const uint32_t ml = (SAH && segs) ? segs[codes[li] >> meshShift].maxLeaf : maxLeaf;
+    uint32_t self = kLeafBit | (uint32_t)li;
+    BoxF mine = leafBoxes[sortedIds[li]];
+    float cost[8];
+    if(SAH)
+    {
+        const float leafCost = cPrim * box_cost_area(mine);
+        for(int i = 0; i < 8; i++) cost[i] = leafCost;
+    }
     for(int guard = 0; p != kNoParent; guard++)
     {
         if(p >= nInt || guard > n) { atomicOr(errorFlag, 1u); return; }
+        const uint4 nd = __ldg(reinterpret_cast<const uint4*>(nodes + p));   // left, right, parent, leaf count
         if(atomicAdd(&counters[p], 1u) == 0u) return;
         __threadfence();
-        const uint32_t ch[2] = { nodes[p].left, nodes[p].right };
-        for(int c = 0; c < 2; c++)
+        const bool left = nd.x == self;
+        const uint32_t other = left ? nd.y : nd.x;
+        const uint32_t ix = other & ~kLeafBit;
+        if((!left && nd.y != self) || ix >= ((other & kLeafBit) ? (uint32_t)n : nInt)) { atomicOr(errorFlag, 1u); return; }
+        BoxF sib;
+        float sibCost[8];
+        if(other & kLeafBit)
         {
-            const bool leaf = (ch[c] & kLeafBit) != 0u;
-            const uint32_t ix = ch[c] & ~kLeafBit;
-            if((leaf && ix >= (uint32_t)n) || (!leaf && ix >= nInt)) { atomicOr(errorFlag, 1u); return; }
-        }
-        float cl[8], cr[8];
-        for(int i = 0; i < 8; i++)
-        {
-            cl[i] = ref_cost(costs, leafBoxes, sortedIds, ch[0], i + 1, cPrim);
-            cr[i] = ref_cost(costs, leafBoxes, sortedIds, ch[1], i + 1, cPrim);
-        }
-        WideCost w;
-        float d[8];
-        uint8_t kd[8];
-        d[0] = __int_as_float(0x7f800000);
-        kd[0] = 0;
-        for(int i = 2; i <= 8; i++)
-        {
-            float best = __int_as_float(0x7f800000);
-            int bk = 1;
-            for(int k = 1; k < i; k++)
+            sib = leafBoxes[sortedIds[ix]];
+            if(SAH)
             {
-                const float v = cl[k - 1] + cr[i - k - 1];
-                if(v < best) { best = v; bk = k; }
+                const float leafCost = cPrim * box_cost_area(sib);
+                for(int i = 0; i < 8; i++) sibCost[i] = leafCost;
             }
-            d[i - 1] = best;
-            kd[i - 1] = (uint8_t)bk;
         }
-        const BoxF b = nodeBoxes[p];
-        const float dx = b.mx[0] - b.mn[0], dy = b.mx[1] - b.mn[1], dz = b.mx[2] - b.mn[2];
-        const float area = dx * dy + dy * dz + dz * dx;
-        const uint32_t cnt = nodes[p].leafCount;
-        const float cInt = cNode * area + d[7];
-        const float cLeaf = cPrim * (float)cnt * area;
-        w.asLeaf = (cnt <= ml && cLeaf <= cInt) ? 1u : 0u;
-        w.c[0] = w.asLeaf ? cLeaf : cInt;
-        w.split[0] = 0;
-        for(int i = 2; i <= 8; i++)
+        else
         {
-            if(d[i - 1] < w.c[i - 2]) { w.c[i - 1] = d[i - 1]; w.split[i - 1] = kd[i - 1]; }
-            else { w.c[i - 1] = w.c[i - 2]; w.split[i - 1] = 0; }
+            const float2* src = reinterpret_cast<const float2*>(&nodeBoxes[ix]);
+            const float2 a = __ldcg(src), b = __ldcg(src + 1), c = __ldcg(src + 2);
+            if(SAH)
+            {
+                const float4 c0 = __ldcg(reinterpret_cast<const float4*>(costs[ix].c));
+                const float4 c1 = __ldcg(reinterpret_cast<const float4*>(costs[ix].c) + 1);
+                sibCost[0] = c0.x; sibCost[1] = c0.y; sibCost[2] = c0.z; sibCost[3] = c0.w;
+                sibCost[4] = c1.x; sibCost[5] = c1.y; sibCost[6] = c1.z; sibCost[7] = c1.w;
+            }
+            sib.mn[0] = a.x; sib.mn[1] = a.y; sib.mn[2] = b.x;
+            sib.mx[0] = b.y; sib.mx[1] = c.x; sib.mx[2] = c.y;
         }
-        w.fullSplit = kd[7];
-        costs[p] = w;
+        BoxF b;
+        for(int k = 0; k < 3; k++)
+        {
+            b.mn[k] = fminf(fminf(FLT_MAX, left ? mine.mn[k] : sib.mn[k]), left ? sib.mn[k] : mine.mn[k]);
+            b.mx[k] = fmaxf(fmaxf(-FLT_MAX, left ? mine.mx[k] : sib.mx[k]), left ? sib.mx[k] : mine.mx[k]);
+        }
+        mine = b;
+        nodeBoxes[p] = b;
+        if(SAH)
+        {
+            float cl[8], cr[8];
+            for(int i = 0; i < 8; i++)
+            {
+                cl[i] = left ? cost[i] : sibCost[i];
+                cr[i] = left ? sibCost[i] : cost[i];
+            }
+            WideCost w;
+            float d[8];
+            uint8_t kd[8];
+            d[0] = __int_as_float(0x7f800000);
+            kd[0] = 0;
+#pragma unroll
+            for(int i = 2; i <= 8; i++)
+            {
+                float best = __int_as_float(0x7f800000);
+                int bk = 1;
+#pragma unroll
+                for(int k = 1; k < i; k++)
+                {
+                    const float v = cl[k - 1] + cr[i - k - 1];
+                    if(v < best) { best = v; bk = k; }
+                }
+                d[i - 1] = best;
+                kd[i - 1] = (uint8_t)bk;
+            }
+            const float area = box_cost_area(b);
+            const uint32_t cnt = nd.w;
+            const float cInt = cNode * area + d[7];
+            const float cLeaf = cPrim * (float)cnt * area;
+            w.asLeaf = (cnt <= ml && cLeaf <= cInt) ? 1u : 0u;
+            w.c[0] = w.asLeaf ? cLeaf : cInt;
+            w.split[0] = 0;
+#pragma unroll
+            for(int i = 2; i <= 8; i++)
+            {
+                if(d[i - 1] < w.c[i - 2]) { w.c[i - 1] = d[i - 1]; w.split[i - 1] = kd[i - 1]; }
+                else { w.c[i - 1] = w.c[i - 2]; w.split[i - 1] = 0; }
+            }
+            w.fullSplit = kd[7];
+            costs[p] = w;
+            for(int i = 0; i < 8; i++) cost[i] = w.c[i];
+        }
         __threadfence();
-        p = nodes[p].parent;
+        self = p;
+        p = nd.z;
     }
 }
 
@@ -590,7 +593,7 @@ struct CollapseArgs
     uint32_t*       counters;   // kCtr*: nodes, leaf payloads, error, then a queue size per level
     uint32_t        leafCount;  // leaves (payload capacity)
     uint32_t        wideCap;    // wide node / queue capacity
-    const WideCost* costs;      // SAH-optimal collapse choices (k_wide_cost), or null: greedy
+    const WideCost* costs;      // SAH-optimal collapse choices (k_bottom_up), or null: greedy
     uint32_t        sahMaxLeaf; // the choices apply to wide nodes whose leaf size is at most this
 };
 
@@ -975,7 +978,7 @@ inline unsigned gridFor(uint32_t n, int tpb = kTPB) { return (unsigned)((n + tpb
 
 namespace {
 // Collapse of the binary tree to 8-wide nodes, MRG_BVH_COLLAPSE: "sah" the
-// SAH-optimal one (k_wide_cost) everywhere, "sah-blas" for BLASes only,
+// SAH-optimal one (k_bottom_up) everywhere, "sah-blas" for BLASes only,
 // "sah-large" only for BLASes with one triangle per leaf child, "greedy" the
 // largest-child-first expansion everywhere; the default is "sah-blas".
 // MRG_BVH_SAH_CPRIM / MRG_BVH_SAH_CINST are the costs of a triangle test and
@@ -1217,17 +1220,10 @@ bool build_wide_bvh(const BuildInput& in, BuildResult& out, BuildWorkspace& ws, 
         k_karras<<<gridFor(n - 1), kTPB, 0, st>>>(kb.Current(), (int)n, dNodes, dLeafParent, nullptr, 0u, nullptr);
         MRG_CK(cudaGetLastError());
         MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
-        k_bottom_up<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes,
-                                                 dNodeBoxes, dCnt, (int)n, dCounters + kCtrError);
+        (sah ? k_bottom_up<true> : k_bottom_up<false>)<<<gridFor(n), kTPB, 0, st>>>(
+            dLeafParent, vb.Current(), dLeafBoxes, dNodes, dNodeBoxes, dCosts, dCnt, (int)n, nullptr, 0u, nullptr, in.maxLeaf,
+            1.0f, in.kind == 1 ? sah_cinst() : sah_cprim(), dCounters + kCtrError);
         MRG_CK(cudaGetLastError());
-        if(sah)
-        {
-            MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
-            k_wide_cost<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes, dNodeBoxes,
-                                                     dCosts, dCnt, (int)n, nullptr, nullptr, 0u, in.maxLeaf, 1.0f,
-                                                     in.kind == 1 ? sah_cinst() : sah_cprim(), dCounters + kCtrError);
-            MRG_CK(cudaGetLastError());
-        }
         MRG_CK(cudaMemcpyAsync(&rootBox, dNodeBoxes, sizeof(BoxF), cudaMemcpyDeviceToHost, st));
         rootItem = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -1356,20 +1352,14 @@ bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, TriRecord* 
     {
         MRG_CK(cudaMemsetAsync(dNodes, 0xFF, sizeof(BinNode) * nInt, st));
         MRG_CK(cudaMemsetAsync(dLeafParent, 0xFF, sizeof(uint32_t) * n, st));
-        k_karras<<<gridFor(n - 1), kTPB, 0, st>>>(kb.Current(), (int)n, dNodes, dLeafParent, dFirsts, M, dMeshRoot);
+        k_karras<<<gridFor(n - 1), kTPB, 0, st>>>(kb.Current(), (int)n, dNodes, dLeafParent, dFirsts, 3u * bits,
+                                                  dMeshRoot);
         MRG_CK(cudaGetLastError());
         MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
-        k_bottom_up<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes,
-                                                 dNodeBoxes, dCnt, (int)n, dCounters + kCtrError);
+        (sah ? k_bottom_up<true> : k_bottom_up<false>)<<<gridFor(n), kTPB, 0, st>>>(
+            dLeafParent, vb.Current(), dLeafBoxes, dNodes, dNodeBoxes, dCosts, dCnt, (int)n, kb.Current(), 3u * bits, dSegs, 3u,
+            1.0f, sah_cprim(), dCounters + kCtrError);
         MRG_CK(cudaGetLastError());
-        if(sah)
-        {
-            MRG_CK(cudaMemsetAsync(dCnt, 0, sizeof(uint32_t) * nInt, st));
-            k_wide_cost<<<gridFor(n), kTPB, 0, st>>>(dLeafParent, vb.Current(), dLeafBoxes, dNodes, dNodeBoxes,
-                                                     dCosts, dCnt, (int)n, dFirsts, dSegs, M, 3u, 1.0f,
-                                                     sah_cprim(), dCounters + kCtrError);
-            MRG_CK(cudaGetLastError());
-        }
     }
     k_mesh_boxes<<<gridFor(M), kTPB, 0, st>>>(dMeshRoot, M, dNodeBoxes, dLeafBoxes, vb.Current(), n, dMeshBoxes,
                                               dSegs, dQ[0], dCounters + kCtrError);
