@@ -353,9 +353,11 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t nAll = L.nLights + (L.env.enabled ? 1u : 0u);
     const float invN = nAll ? __fdiv_rn(1.0f, (float)nAll) : 0.0f;
-    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
-    for(uint32_t base = first; base < n; base += stride)
+    // block-uniform trip count: every thread reaches the appends
+    uint32_t turn = 0;
+    for(uint32_t tile = blockIdx.x * blockDim.x; tile < n; tile += stride, turn++)
     {
+        const uint32_t base = tile + (threadIdx.x & ~31u);
         bool alive = false, shadow = false;
         uint32_t i = 0;
         if(work_item(W, base, i))
@@ -576,8 +578,7 @@ k_shade_guided(PtLaunch L, PtPaths P, GuideGrid G, GuidePaths Q, PtSceneTables T
                 }
             }
         }
-        warp_append(alive, i, nextList, nextCount);
-        warp_append(shadow, i, P.shadowList, shadowCount);
+        block_append<kGuideTPB>(turn, i, alive, nextList, nextCount, shadow, P.shadowList, shadowCount);
     }
 }
 

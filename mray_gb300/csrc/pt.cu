@@ -73,12 +73,15 @@ k_raygen(PtLaunch L, PtPaths P, uint32_t* aliveList)
 // ---------------------------------------------------------------------------
 // Shade: light hits (emission with MIS), misses (skysphere with MIS), surface
 // hits (NEE + BxDF sample + Russian roulette).  Live paths and shadow rays
-// are appended to their lists with one atomic per warp.  NC colour channels:
-// 3 (RGB) or 4 (wavelengths); AM a PtAdjointMode.
+// are appended to their lists with one atomic per block: per warp they were
+// 130,000 a list in a bounce of 4M paths, on two words (1080p production frame
+// 16.24 -> 15.95 ms, box scene 834 -> 802 us).  NC colour channels: 3 (RGB) or
+// 4 (wavelengths); AM a PtAdjointMode; BLOCKS: resident blocks an SM that the
+// registers allow for (pt_shade_impl).
 // ---------------------------------------------------------------------------
 
-template<bool SPEC, uint32_t AM, int CM>
-__global__ void __launch_bounds__(kPtTPB)
+template<bool SPEC, uint32_t AM, int CM, int BLOCKS>
+__global__ void __launch_bounds__(kPtTPB, BLOCKS)
 k_shade(PtLaunch L, PtPaths P, PtSceneTables T, PtWork W, uint32_t* nextList, uint32_t* nextCount,
         uint32_t* shadowCount)
 {
@@ -94,10 +97,11 @@ k_shade(PtLaunch L, PtPaths P, PtSceneTables T, PtWork W, uint32_t* nextList, ui
     const uint32_t nAll = L.nLights + (L.env.enabled ? 1u : 0u);
     const float invN = nAll ? __fdiv_rn(1.0f, (float)nAll) : 0.0f;
     EmisRun emis{ kNoEmission, 0.0f, 0.0f, 0.0f };
-    // warp-uniform trip count so every lane reaches the ballots
-    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
-    for(uint32_t base = first; base < n; base += stride)
+    // block-uniform trip count: every thread reaches the appends
+    uint32_t turn = 0;
+    for(uint32_t tile = blockIdx.x * blockDim.x; tile < n; tile += stride, turn++)
     {
+        const uint32_t base = tile + (threadIdx.x & ~31u);
         bool alive = false, shadow = false, query = false;
         uint32_t i = 0;
         if(work_item(W, base, i))
@@ -172,6 +176,7 @@ k_shade(PtLaunch L, PtPaths P, PtSceneTables T, PtWork W, uint32_t* nextList, ui
                             }
                         }
                     }
+                    P.rad[i] = f4(rad);          // a surface leaves it as it is
                 }
                 else
                 {
@@ -303,7 +308,6 @@ k_shade(PtLaunch L, PtPaths P, PtSceneTables T, PtWork W, uint32_t* nextList, ui
                     }
                     }   // not terminal
                 }
-                P.rad[i] = f4(rad);
             }
             else if(hk.x == kMissMark && L.env.enabled)
             {
@@ -324,8 +328,7 @@ k_shade(PtLaunch L, PtPaths P, PtSceneTables T, PtWork W, uint32_t* nextList, ui
                 }
             }
         }
-        warp_append(alive, i, nextList, nextCount);
-        warp_append(shadow, i, P.shadowList, shadowCount);
+        block_append<kPtTPB>(turn, i, alive, nextList, nextCount, shadow, P.shadowList, shadowCount);
         if(CM == 1) warp_append(query, i, L.cache.queryList, L.cache.queryCount);
     }
     if(ADJ && L.adj.gradEmission) emis_flush(emis, L.adj.gradEmission);
@@ -651,13 +654,21 @@ cudaError_t pt_shade_impl(const PtLaunch& L, const PtPaths& P, const PtSceneTabl
 {
     // a group's last warp may be partly empty, so up to 32 lanes more a list
     const unsigned grid = grid_for(L.slots + 32u * W.nLists, smCount);
+    // Two blocks an SM (114-120 registers) where a launch is short, three (80, 200
+    // bytes spilled) where it runs long enough for more loads in flight to pay:
+    // 4M paths a pass 15.91 -> 15.24 ms (production), 12.16 -> 11.70 (gradients);
+    // 334k and 524k even (757 / 759, 801 / 800 us), 14k 170 -> 175 us.
+    const bool wide = L.slots >= (1u << 20);
 #define MRG_SHADE(...) k_shade<__VA_ARGS__><<<grid, kPtTPB, 0, st>>>(L, P, T, W, nextList, nextCount, shadowCount)
-    if(L.cache.mode == 1u && L.spec.enabled) MRG_SHADE(true, kAdjOff, 1);
-    else if(L.cache.mode == 1u) MRG_SHADE(false, kAdjOff, 1);
-    else if(L.adj.mode == kAdjRecord) MRG_SHADE(false, kAdjRecord, 0);
-    else if(L.adj.mode == kAdjReplay) MRG_SHADE(false, kAdjReplay, 0);
-    else if(L.spec.enabled) MRG_SHADE(true, kAdjOff, 0);
-    else MRG_SHADE(false, kAdjOff, 0);
+    if(L.cache.mode == 1u && L.spec.enabled) MRG_SHADE(true, kAdjOff, 1, 2);
+    else if(L.cache.mode == 1u) MRG_SHADE(false, kAdjOff, 1, 2);
+    else if(L.adj.mode == kAdjReplay) MRG_SHADE(false, kAdjReplay, 0, 2);
+    else if(L.adj.mode == kAdjRecord && wide) MRG_SHADE(false, kAdjRecord, 0, 3);
+    else if(L.adj.mode == kAdjRecord) MRG_SHADE(false, kAdjRecord, 0, 2);
+    else if(L.spec.enabled && wide) MRG_SHADE(true, kAdjOff, 0, 3);
+    else if(L.spec.enabled) MRG_SHADE(true, kAdjOff, 0, 2);
+    else if(wide) MRG_SHADE(false, kAdjOff, 0, 3);
+    else MRG_SHADE(false, kAdjOff, 0, 2);
 #undef MRG_SHADE
     return cudaGetLastError();
 }

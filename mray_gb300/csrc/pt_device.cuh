@@ -711,6 +711,32 @@ __device__ __forceinline__ void warp_append(bool pred, uint32_t value, uint32_t*
     if(pred) list[base + __popc(m & ((1u << lane) - 1u))] = value;
 }
 
+// Appends to two lists for a whole block of TPB: one atomic a list and call.
+// Every thread of the block calls it, with `turn` alternating between calls.
+template<uint32_t TPB>
+__device__ __forceinline__ void block_append(uint32_t turn, uint32_t value, bool a, uint32_t* listA, uint32_t* countA,
+                                             bool b, uint32_t* listB, uint32_t* countB)
+{
+    constexpr uint32_t kWarps = TPB / 32;
+    __shared__ uint32_t sCount[2][2][kWarps], sBase[2][2];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, t = turn & 1u;
+    const uint32_t ma = __ballot_sync(0xFFFFFFFFu, a), mb = __ballot_sync(0xFFFFFFFFu, b);
+    if(lane < 2u) sCount[t][lane][warp] = __popc(lane ? mb : ma);
+    __syncthreads();
+    if(threadIdx.x < 2u)
+    {
+        uint32_t n = 0;
+        for(uint32_t w = 0; w < kWarps; w++) n += sCount[t][threadIdx.x][w];
+        sBase[t][threadIdx.x] = n ? atomicAdd(threadIdx.x ? countB : countA, n) : 0u;
+    }
+    __syncthreads();
+    uint32_t atA = sBase[t][0], atB = sBase[t][1];
+    for(uint32_t w = 0; w < warp; w++) { atA += sCount[t][0][w]; atB += sCount[t][1][w]; }
+    const uint32_t lt = (1u << lane) - 1u;
+    if(a) listA[atA + __popc(ma & lt)] = value;
+    if(b) listB[atB + __popc(mb & lt)] = value;
+}
+
 // Items of a shade kernel's work: the lists one after another, each padded to
 // whole warps so that no warp holds two groups.
 __device__ __forceinline__ uint32_t work_size(const PtWork& W)
