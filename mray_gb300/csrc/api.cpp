@@ -79,8 +79,8 @@ void free_accel(mrg_ctx* c)
     cudaFree(c->dNodes); c->dNodes = nullptr;
     cudaFree(c->dTris); c->dTris = nullptr;
     cudaFree(c->dInsts); c->dInsts = nullptr;
-    cudaFree(c->dTlasLeaf); c->dTlasLeaf = nullptr;
-    c->capNodes = c->capTris = c->capInsts = c->capTlasLeaf = 0;
+    cudaFree(c->dInstSlot); c->dInstSlot = nullptr;
+    c->capNodes = c->capTris = c->capInsts = c->capInstSlot = 0;
     c->blasNodes = c->blasTris = c->tlasNodes = 0;
     c->scene = mrg::TraceScene{};
     c->built = false;
@@ -433,7 +433,7 @@ mrg_status mrg_build(mrg_ctx* c)
     totalNodes += tlas.nodeCount;
     e = ensure(c->dNodes, c->capNodes, mrg::kWideNodeBytes * totalNodes);
     if(e == cudaSuccess) e = ensure(c->dInsts, c->capInsts, sizeof(mrg::HostInstRecord) * ni);
-    if(e == cudaSuccess) e = ensure(c->dTlasLeaf, c->capTlasLeaf, sizeof(uint32_t) * ni);
+    if(e == cudaSuccess) e = ensure(c->dInstSlot, c->capInstSlot, sizeof(uint32_t) * ni);
     uint64_t nodeOff = 0, triOff = 0;
     std::vector<uint64_t> pieceNodeOff(pieces.size());
     for(size_t pi = 0; pi < pieces.size() && e == cudaSuccess; pi++)
@@ -456,8 +456,6 @@ mrg_status mrg_build(mrg_ctx* c)
                                 static_cast<char*>(c->dNodes) + mrg::kWideNodeBytes * tlasOff),
                             tlas.nodeCount, (uint32_t)tlasOff, 0u, st))
         e = cudaErrorLaunchFailure;
-    if(e == cudaSuccess)
-        e = cudaMemcpyAsync(c->dTlasLeaf, tlas.leafIds, sizeof(uint32_t) * ni, cudaMemcpyDeviceToDevice, st);
     std::vector<mrg::HostInstRecord> recs(ni);
     for(int k = 0; k < 3; k++) { c->sceneBoxExact[k] = 3.0e38f; c->sceneBoxExact[3 + k] = -3.0e38f; }
     for(uint32_t i = 0; i < ni; i++)
@@ -479,8 +477,13 @@ mrg_status mrg_build(mrg_ctx* c)
         }
         recs[i].wmin[3] = 0.0f; recs[i].wmax[3] = 0.0f;
     }
+    void* dRecs = nullptr;
+    if(e == cudaSuccess) e = ws.take(&dRecs, sizeof(mrg::HostInstRecord) * ni);
     if(e == cudaSuccess)
-        e = cudaMemcpyAsync(c->dInsts, recs.data(), sizeof(mrg::HostInstRecord) * ni, cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync(dRecs, recs.data(), sizeof(mrg::HostInstRecord) * ni, cudaMemcpyHostToDevice, st);
+    if(e == cudaSuccess && !mrg::place_instances(static_cast<const mrg::InstRecord*>(dRecs), tlas.leafIds, ni,
+                                                 static_cast<mrg::InstRecord*>(c->dInsts), c->dInstSlot, st))
+        e = cudaErrorLaunchFailure;
     if(e == cudaSuccess) e = cudaStreamSynchronize(st);
     if(e != cudaSuccess) return cuda_failed(e, "mrg_build: placement");
 
@@ -490,7 +493,7 @@ mrg_status mrg_build(mrg_ctx* c)
     c->scene.nodes = static_cast<const mrg::WideNode*>(c->dNodes);
     c->scene.tris = static_cast<const mrg::TriRecord*>(c->dTris);
     c->scene.insts = static_cast<const mrg::InstRecord*>(c->dInsts);
-    c->scene.tlasLeaf = c->dTlasLeaf;
+    c->scene.instSlot = c->dInstSlot;
     c->scene.tlasRoot = (uint32_t)tlasOff;
     c->scene.instCount = ni;
     c->scene.nodeCount = (uint32_t)totalNodes;

@@ -970,6 +970,19 @@ __global__ void k_relocate(const WideNode* __restrict__ in, WideNode* __restrict
     out[i] = w;
 }
 
+// Six lanes an instance record, 16 bytes each.
+__global__ void k_place_instances(const uint4* __restrict__ in, const uint32_t* __restrict__ leafIds, uint32_t n,
+                                  uint4* __restrict__ out, uint32_t* __restrict__ slotOf)
+{
+    constexpr uint32_t kParts = sizeof(InstRecord) / sizeof(uint4);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, k = t / kParts, part = t % kParts;
+    if(k >= n) return;
+    const uint32_t id = leafIds[k];
+    if(id >= n) return;
+    out[(size_t)k * kParts + part] = in[(size_t)id * kParts + part];
+    if(part == 0u) slotOf[id] = k;
+}
+
 inline unsigned gridFor(uint32_t n, int tpb = kTPB) { return (unsigned)((n + tpb - 1) / tpb); }
 
 #define MRG_CK(x) do { cudaError_t e_ = (x); if(e_ != cudaSuccess) { err = std::string(#x) + ": " + cudaGetErrorString(e_); goto fail; } } while(0)
@@ -1393,6 +1406,15 @@ fail:
     cudaStreamSynchronize(st);
     out = BatchResult{};
     return false;
+}
+
+bool place_instances(const InstRecord* in, const uint32_t* leafIds, uint32_t n, InstRecord* out, uint32_t* slotOf,
+                     cudaStream_t st)
+{
+    if(n == 0) return true;
+    k_place_instances<<<gridFor(n * 6u), kTPB, 0, st>>>(reinterpret_cast<const uint4*>(in), leafIds, n,
+                                                        reinterpret_cast<uint4*>(out), slotOf);
+    return cudaGetLastError() == cudaSuccess;
 }
 
 bool relocate_nodes(const WideNode* src, WideNode* dst, uint32_t n, uint32_t nodeOff,

@@ -77,6 +77,9 @@ struct BatchResult
 // The triangle records go straight to `tris` (one per triangle).
 bool build_wide_bvh_batch(const std::vector<BatchMeshInput>& meshes, TriRecord* tris, BatchResult& out,
                           BuildWorkspace& ws, cudaStream_t st, std::string& err);
+// Instance records from the order of their numbers to that of the TLAS leaves (leafIds).
+bool place_instances(const InstRecord* in, const uint32_t* leafIds, uint32_t n, InstRecord* out, uint32_t* slotOf,
+                     cudaStream_t st);
 bool relocate_nodes(const WideNode* src, WideNode* dst, uint32_t n, uint32_t nodeOff,
                     uint32_t triOff, cudaStream_t st);
 
@@ -86,7 +89,7 @@ struct TraceScene
     const WideNode*   nodes = nullptr;     // all BLAS nodes then TLAS nodes
     const TriRecord*  tris = nullptr;
     const InstRecord* insts = nullptr;
-    const uint32_t*   tlasLeaf = nullptr;  // instance id per TLAS payload slot
+    const uint32_t*   instSlot = nullptr;  // an instance's place among the records (TLAS leaf order)
     uint32_t          tlasRoot = 0;
     uint32_t          instCount = 0;
     uint32_t          nodeCount = 0;       // bounds for every index read from the tree

@@ -80,12 +80,12 @@ struct mrg_ctx
     bool built = false;
 
     // accelerator (device); a rebuild of about the same size keeps the arrays
-    size_t    capNodes = 0, capTris = 0, capInsts = 0, capTlasLeaf = 0;   // bytes
+    size_t    capNodes = 0, capTris = 0, capInsts = 0, capInstSlot = 0;   // bytes
     mrg::BuildWorkspace buildWs;
     void*     dNodes = nullptr;
     void*     dTris = nullptr;
     void*     dInsts = nullptr;
-    uint32_t* dTlasLeaf = nullptr;
+    uint32_t* dInstSlot = nullptr;
     uint64_t  blasNodes = 0, blasTris = 0, tlasNodes = 0;
     mrg::TraceScene scene;
     float     sceneBox[6] = { 0, 0, 0, 0, 0, 0 };        // conservative (TLAS) box

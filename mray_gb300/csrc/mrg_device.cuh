@@ -7,8 +7,11 @@
 //                        e0/e1 are the exact float differences MRay's
 //                        Moller-Trumbore forms first (Source/Core/Ray.hpp:131-132),
 //                        so storing them keeps the test bit-identical.
-//   InstRecord insts[]   96 B each: inverse 3x4 transform rows, keys, exact world AABB.
-//   uint32    tlasLeaf[] instance index per TLAS leaf slot.
+//   InstRecord insts[]   96 B each: inverse 3x4 transform rows, keys, exact world
+//                        AABB, in the order of the TLAS leaves: a list of instance
+//                        numbers between the two was a load more in the chain of
+//                        every instance test (3.95M rays 1,732 -> 1,701 us).
+//   uint32    instSlot[] place of every instance in insts.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

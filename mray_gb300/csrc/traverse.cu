@@ -312,7 +312,8 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
                     live = true;
                     if(LOCAL)
                     {
-                        const uint32_t inst = __ldg(instIds + i);
+                        const uint32_t id = __ldg(instIds + i);
+                        const uint32_t inst = id < sc.instCount ? __ldg(sc.instSlot + id) : kInvalidIndex;
                         if(inst >= sc.instCount) { atomicOr(scr.errorFlag, kTraceBadIndex); live = false; }
                         else
                         {
@@ -448,9 +449,7 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
                     for(uint32_t cand = tg.y; cand != 0u; cand &= cand - 1u)
                     {
                         const uint32_t bt = __ffs(cand) - 1u;
-                        const uint32_t pi = tg.x + bt;
-                        if(pi >= sc.instCount) { atomicOr(scr.errorFlag, kTraceBadIndex); finished = true; break; }
-                        const uint32_t inst = __ldg(sc.tlasLeaf + pi);
+                        const uint32_t inst = tg.x + bt;      // records lie in leaf order
                         if(inst >= sc.instCount) { atomicOr(scr.errorFlag, kTraceBadIndex); finished = true; break; }
                         const float4* ip = reinterpret_cast<const float4*>(sc.insts + inst);
                         float tEnter;
@@ -467,7 +466,7 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
                     if(best != 32u)
                     {
                         keep &= ~(1u << best);
-                        const uint32_t inst = __ldg(sc.tlasLeaf + tg.x + best);
+                        const uint32_t inst = tg.x + best;
                         const float4* ip = reinterpret_cast<const float4*>(sc.insts + inst);
                         if(ng.y > 0x00FFFFFFu)
                         {
