@@ -560,8 +560,8 @@ def c2_scene_pt(args, dev):
 
 def c3_adjoint(args, dev):
     """Differentiable workload: box + 65,024-triangle textured sphere, 512^2
-    f32 albedo texture, 512^2 image, 32 spp, depth 6; one path-replay adjoint
-    (primal + replay) per step giving d(loss)/d(texture) and d(loss)/d(area-light
+    f32 albedo texture, 512^2 image, 32 spp, depth 6; one adjoint call per
+    step giving d(loss)/d(texture) and d(loss)/d(area-light
     emission)."""
     import torch
     from mray_gb300.pt import PathTracer

@@ -363,17 +363,18 @@ mrg_status mrg_pt_generate_mips(mrg_ctx* ctx, uint32_t texture_id, float filter_
  * level, and every level up to it must be given (else the next render fails). */
 mrg_status mrg_pt_set_texture_mip(mrg_ctx* ctx, uint32_t texture_id, uint32_t level, const void* texels);
 
-/* ---- Path-replay adjoint (no reference counterpart) ---------------------- */
+/* ---- Adjoint (no reference counterpart) ----------------------------------- */
 /* Gradient of  sum_pixels <d_image_adjoint[p].rgb, I[p].rgb>  with respect to
  * the RGB texels of f32 texture texture_id (a Lambert albedo) and to the RGB
  * radiance of every area light, I being the image of params (RGB mode):
- * I[p] = (sum of the pixel's spp sample radiances) / spp.  Each pass runs
- * twice with the same paths (counter-based random numbers): the primal records
- * every path's radiance, the replay adds at every vertex on the texture
- * d * (radiance after the vertex) / albedo  into the four texels of its
- * bilinear read (Vicini et al. 2021, "Path Replay Backpropagation"), and, for
- * every emission it gathers (a light hit, or a visible NEE sample), d * (the
- * contribution / the light's radiance) into the light's instance.
+ * I[p] = (sum of the pixel's spp sample radiances) / spp.  Every vertex on the
+ * texture adds  d * (radiance after the vertex) / albedo  into the four texels
+ * of its bilinear read, and every emission that is gathered (a light hit, or a
+ * visible NEE sample) d * (the contribution / the light's radiance) into the
+ * light's instance.  A pass keeps its vertices on the texture until its paths
+ * have ended; where they would take more than 4 GiB (samplesPerPass * pixels *
+ * maxDepth * 40 bytes, per pipeline) it runs a second time with the same paths
+ * instead (Vicini et al. 2021, "Path Replay Backpropagation").
  * d_grad (RGBA f32 per texel, A unused) and d_grad_emission (RGBA f32 per
  * instance, A unused; entries of instances that are not area lights stay
  * untouched) are ADDED to (atomics).  texture_id = MRG_PT_NO_TEXTURE asks for

@@ -1,4 +1,4 @@
-"""Differentiable rendering through the path-replay adjoint.
+"""Differentiable rendering through the adjoint.
 
 ``render_albedo(texture, tracer, tex_id, params)`` returns the rendered image
 (weight-normalised RGB, (H, W, 3)) as a function of an f32 RGBA albedo
@@ -7,8 +7,9 @@ tensor).  ``render_scene(texture, emission, tracer, tex_id, lights, params)``
 is the same image as a function of the texture and of the RGB radiance of the
 area-light instances ``lights`` ((len(lights), 3); the forward pass sets them
 on the tracer).  Their backward pass is ``mrg_pt_adjoint``: the image gradient
-goes in as dLoss/dPixel and the texture (and emission) gradients come out,
-recomputing every path from its sample index instead of storing it.  Russian
+goes in as dLoss/dPixel and the texture (and emission) gradients come out;
+every path is traced again from its sample index, nothing of it is kept from
+the forward pass.  Russian
 roulette's throughput-dependent probability is a constant to the adjoint, so
 gradient checks render with ``rr_start == max_depth``.
 """

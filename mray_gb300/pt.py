@@ -73,7 +73,7 @@ class PathTracer:
         return image, (l.value if loss else None)
 
     def adjoint(self, p, tex_id, image_adjoint, grad=None, image=None, stream=None, grad_emission=None):
-        """Path-replay adjoint (see mrg_pt_adjoint): image_adjoint is a
+        """Adjoint (see mrg_pt_adjoint): image_adjoint is a
         (h, w, 4) float32 CUDA tensor of dLoss/dPixel; returns grad, a
         (texH, texW, 4) float32 CUDA tensor the texture gradient is added to
         (None when tex_id is None: emission only).  grad_emission, a
