@@ -1,7 +1,7 @@
 """The traversal's half-precision node test (traverse.cu: intersect_node) never
 culls a child box that the ray meets: numpy restates the builder's plane
 quantisation and the test, halves rounded as the GPU rounds them, and a
-64-bit slab test of the boxes before padding is the judge."""
+64-bit slab test of the boxes before padding decides."""
 import numpy as np
 import pytest
 
