@@ -118,7 +118,7 @@ __device__ __forceinline__ void sh16(float x, float y, float z, float* o)
 // differ in low bits only), which makes it one lookup.  Then they trade
 // values, so that each lane has one of two levels whole and sums its corners
 // in the order of one lane per level.  2,073,600 samples, 16 levels of 2^19:
-// 905 -> 598 us.
+// 905 -> 598 us (583 with the CTAs of nrc_query).
 __device__ void encode_pair(const NrcState& S, const float4* in, bool valid, uint32_t cx, uint16_t* row)
 {
     const NrcGrid& G = S.grid;
@@ -193,7 +193,8 @@ __device__ void encode_pair(const NrcState& S, const float4* in, bool valid, uin
 // Forward: inference (out) or training (stores activations and outputs)
 // ---------------------------------------------------------------------------
 // WARPS warps per CTA share one shared-memory copy of the weights; more warps
-// per CTA keep more hash-grid gathers in flight per SM.  (32 samples a warp,
+// per CTA keep more hash-grid gathers in flight per SM and leave more of it to
+// the L1 (see kNrcSmallQuery).  (32 samples a warp,
 // each weight fragment used twice, measured the same: 597 us against 598, the
 // registers cost as many warps as the reads save.)
 template<bool TRAIN, bool LIST, int WARPS>
@@ -234,8 +235,16 @@ k_nrc_forward(NrcState S, const float4* __restrict__ inputs, const uint32_t* __r
             }
         }
     };
-    for(uint32_t base = (blockIdx.x * WARPS + warp) * 16u; base < n; base += gridDim.x * WARPS * 16u)
+    // Tiles of 16 samples, a CTA's side by side; those of the last, partial round
+    // go one to each CTA in turn, so that no SM has them all (160,000 samples, 2.06
+    // rounds: 73 -> 57 us).
+    const uint32_t tiles = (n + 15u) / 16u, round = gridDim.x * WARPS;
+    for(uint32_t first = 0; first < tiles; first += round)
     {
+        const uint32_t left = tiles - first;
+        const uint32_t mine = left >= round ? blockIdx.x * WARPS + warp : warp * gridDim.x + blockIdx.x;
+        if(mine >= left) break;
+        const uint32_t base = (first + mine) * 16u;
         // ---- encode 16 samples ----
         {
             const uint32_t s = lane >> 1, e = base + s;
@@ -826,14 +835,16 @@ __global__ void k_copy_params(const float* __restrict__ w, uint16_t* __restrict_
 }
 
 #ifndef MRG_NRC_QUERY_WARPS
-#define MRG_NRC_QUERY_WARPS 16       // warps per CTA of the inference forward
+#define MRG_NRC_QUERY_WARPS 32       // warps per CTA of the inference forward
 #endif
 // Queries of up to this many samples take CTAs of 4 warps, which spread over
-// more SMs and stage their weights sooner: 1,000 samples 10.4 us against 16.6,
-// 20,000 14.6 / 16.6, 80,000 35.0 / 39.1, 160,000 61.6 / 62.7, 400,000 135 / 130,
-// 1,000,000 327 / 305.
+// more SMs and stage their weights sooner: 1,000 samples 10.5 us against 26.9,
+// 20,000 14.5 / 26.9, 80,000 33.0 / 34.9, 140,000 53.5 / 47.3, 400,000 133 / 124,
+// 1,000,000 326 / 292.  (One CTA of 32 warps an SM, with one copy of the
+// weights, leaves the L1 48 KB more than two of 16: 2,073,600 samples 583 against
+// 608 us.  The first two levels in that room instead: 609.)
 constexpr int kNrcSmallWarps = 4;
-constexpr uint32_t kNrcSmallQuery = 1u << 17;
+constexpr uint32_t kNrcSmallQuery = 3u << 15;
 constexpr size_t fwd_smem(int warps)
 {
     return (size_t)(kHiddenRows + kNrcOut) * kPad * 2 + (size_t)warps * 16 * kPad * 2;
