@@ -118,7 +118,7 @@ __device__ __forceinline__ void sh16(float x, float y, float z, float* o)
 // differ in low bits only), which makes it one lookup.  Then they trade
 // values, so that each lane has one of two levels whole and sums its corners
 // in the order of one lane per level.  2,073,600 samples, 16 levels of 2^19:
-// 905 -> 598 us (583 with the CTAs of nrc_query).
+// 905 -> 598 us (583 with kNrcWarps).
 __device__ void encode_pair(const NrcState& S, const float4* in, bool valid, uint32_t cx, uint16_t* row)
 {
     const NrcGrid& G = S.grid;
@@ -189,12 +189,29 @@ __device__ void encode_pair(const NrcState& S, const float4* in, bool valid, uin
     }
 }
 
+// The next tile of 16 samples of this warp (its first sample: base), from round
+// `first` on: a CTA's tiles lie side by side; those of the last, partial round
+// go one to each CTA in turn, so that no SM has them all (a query of 160,000
+// samples, 2.06 rounds: 73 -> 57 us) and a small batch is in every SM.
+template<int WARPS>
+__device__ __forceinline__ bool next_tile(uint32_t n, uint32_t& first, uint32_t& base)
+{
+    const uint32_t tiles = (n + 15u) / 16u, round = gridDim.x * WARPS, warp = threadIdx.x >> 5;
+    if(first >= tiles) return false;
+    const uint32_t left = tiles - first;
+    const uint32_t mine = left >= round ? blockIdx.x * WARPS + warp : warp * gridDim.x + blockIdx.x;
+    if(mine >= left) return false;
+    base = (first + mine) * 16u;
+    first += round;
+    return true;
+}
+
 // ---------------------------------------------------------------------------
 // Forward: inference (out) or training (stores activations and outputs)
 // ---------------------------------------------------------------------------
 // WARPS warps per CTA share one shared-memory copy of the weights; more warps
 // per CTA keep more hash-grid gathers in flight per SM and leave more of it to
-// the L1 (see kNrcSmallQuery).  (32 samples a warp,
+// the L1 (kNrcWarps).  (32 samples a warp,
 // each weight fragment used twice, measured the same: 597 us against 598, the
 // registers cost as many warps as the reads save.)
 template<bool TRAIN, bool LIST, int WARPS>
@@ -235,16 +252,8 @@ k_nrc_forward(NrcState S, const float4* __restrict__ inputs, const uint32_t* __r
             }
         }
     };
-    // Tiles of 16 samples, a CTA's side by side; those of the last, partial round
-    // go one to each CTA in turn, so that no SM has them all (160,000 samples, 2.06
-    // rounds: 73 -> 57 us).
-    const uint32_t tiles = (n + 15u) / 16u, round = gridDim.x * WARPS;
-    for(uint32_t first = 0; first < tiles; first += round)
+    for(uint32_t first = 0, base; next_tile<WARPS>(n, first, base);)
     {
-        const uint32_t left = tiles - first;
-        const uint32_t mine = left >= round ? blockIdx.x * WARPS + warp : warp * gridDim.x + blockIdx.x;
-        if(mine >= left) break;
-        const uint32_t base = (first + mine) * 16u;
         // ---- encode 16 samples ----
         {
             const uint32_t s = lane >> 1, e = base + s;
@@ -358,7 +367,7 @@ k_nrc_backward(NrcState S, const float4* __restrict__ inputs, const float4* __re
     const uint32_t g = lane >> 2, t = lane & 3u;
     float* gw = sG + warp * 16 * 33;
     float lossAcc = 0.0f;
-    for(uint32_t base = (blockIdx.x * WARPS + warp) * 16u; base < n; base += gridDim.x * WARPS * 16u)
+    for(uint32_t first = 0, base; next_tile<WARPS>(n, first, base);)
     {
         const uint32_t r0 = base + g, r1 = base + g + 8;
         const bool v0 = r0 < n, v1 = r1 < n;
@@ -834,34 +843,29 @@ __global__ void k_copy_params(const float* __restrict__ w, uint16_t* __restrict_
     }
 }
 
-#ifndef MRG_NRC_QUERY_WARPS
-#define MRG_NRC_QUERY_WARPS 32       // warps per CTA of the inference forward
-#endif
-// Queries of up to this many samples take CTAs of 4 warps, which spread over
-// more SMs and stage their weights sooner: 1,000 samples 10.5 us against 26.9,
-// 20,000 14.5 / 26.9, 80,000 33.0 / 34.9, 140,000 53.5 / 47.3, 400,000 133 / 124,
-// 1,000,000 326 / 292.  (One CTA of 32 warps an SM, with one copy of the
-// weights, leaves the L1 48 KB more than two of 16: 2,073,600 samples 583 against
-// 608 us.  The first two levels in that room instead: 609.)
-constexpr int kNrcSmallWarps = 4;
-constexpr uint32_t kNrcSmallQuery = 3u << 15;
+// Warps per CTA of forward and backward, one CTA an SM: with one copy of the
+// weights in shared memory the L1 keeps 48 KB more than with two CTAs of 16 (a
+// query of 2,073,600 samples 583 against 608 us; the two coarsest levels in that
+// room instead: 609).  Tiles go round the CTAs, so small batches need no smaller
+// CTAs: 1,000 / 20,000 / 40,000 / 160,000 samples 10.4 / 12.8 / 18.5 / 57.0 us, with
+// CTAs of 4 warps 10.4 / 14.4 / 22.6 / 61; a training step of 8,000 / 40,000 / 65,536
+// 158 / 212 / 246 us, with CTAs of 4 warps 158 / 230 / 267.  (80,000 samples, just
+// over a round: 35.0 against 33.0.)
+constexpr int kNrcWarps = 32;
 constexpr size_t fwd_smem(int warps)
 {
     return (size_t)(kHiddenRows + kNrcOut) * kPad * 2 + (size_t)warps * 16 * kPad * 2;
 }
-#ifndef MRG_NRC_TRAIN_WARPS
-#define MRG_NRC_TRAIN_WARPS 4        // warps per CTA of the training forward and backward: a step of 65,536 samples takes
-                                     // 265 us with 4, 261 with 16, 285 with 8; one of 8,000 158, 187, 176
-#endif
 constexpr size_t bwd_smem(int warps)
 {
     return (size_t)kHiddenRows * kPad * 2 + (size_t)kNrcWidth * kPadT4 * 2 + (size_t)warps * 16 * 33 * 4;
 }
 
-template<bool TRAIN, bool LIST, int W>
+template<bool TRAIN, bool LIST>
 cudaError_t launch_forward(const NrcState& S, const float4* in, const uint32_t* list, const uint32_t* nDevice,
                            uint32_t nMax, float4* out, int smCount, cudaStream_t st)
 {
+    constexpr int W = kNrcWarps;
     constexpr size_t smem = fwd_smem(W);
     static int perSMOf[kMaxDevices] = {};          // 0: not configured on that device yet
     int& perSM = perSMOf[launch_device()];
@@ -876,8 +880,7 @@ cudaError_t launch_forward(const NrcState& S, const float4* in, const uint32_t* 
             b = 1;
         perSM = b;
     }
-    const uint32_t tiles = (nMax + 16 * W - 1) / (16 * W);
-    const uint32_t grid = std::max(1u, std::min(tiles, (uint32_t)smCount * (uint32_t)perSM));
+    const uint32_t grid = std::max(1u, std::min((nMax + 15u) / 16u, (uint32_t)smCount * (uint32_t)perSM));
     k_nrc_forward<TRAIN, LIST, W><<<grid, W * 32, smem, st>>>(S, in, list, nDevice, nMax, out);
     return cudaGetLastError();
 }
@@ -913,17 +916,13 @@ void nrc_make_grid(NrcGrid& g, uint32_t levels, uint32_t log2Table, uint32_t bas
 cudaError_t nrc_query(const NrcState& S, const float4* inputs, const uint32_t* nDevice, uint32_t nMax,
                       float4* out, int smCount, cudaStream_t st)
 {
-    return (nMax <= kNrcSmallQuery)
-               ? launch_forward<false, false, kNrcSmallWarps>(S, inputs, nullptr, nDevice, nMax, out, smCount, st)
-               : launch_forward<false, false, MRG_NRC_QUERY_WARPS>(S, inputs, nullptr, nDevice, nMax, out, smCount, st);
+    return launch_forward<false, false>(S, inputs, nullptr, nDevice, nMax, out, smCount, st);
 }
 
 cudaError_t nrc_query_list(const NrcState& S, const float4* inputs, const uint32_t* list, const uint32_t* count,
                            uint32_t nMax, float4* out, int smCount, cudaStream_t st)
 {
-    return (nMax <= kNrcSmallQuery)
-               ? launch_forward<false, true, kNrcSmallWarps>(S, inputs, list, count, nMax, out, smCount, st)
-               : launch_forward<false, true, MRG_NRC_QUERY_WARPS>(S, inputs, list, count, nMax, out, smCount, st);
+    return launch_forward<false, true>(S, inputs, list, count, nMax, out, smCount, st);
 }
 
 cudaError_t nrc_train(NrcState& S, const float4* inputs, const float4* targets, const uint32_t* nDevice,
@@ -944,7 +943,7 @@ cudaError_t nrc_gradients(NrcState& S, const float4* inputs, const float4* targe
                           uint32_t nMax, int smCount, cudaStream_t st)
 {
     if(nMax > S.cap) return cudaErrorInvalidValue;
-    constexpr int W = MRG_NRC_TRAIN_WARPS;
+    constexpr int W = kNrcWarps;
     constexpr size_t bsmem = bwd_smem(W);
     static int perSMOf[kMaxDevices] = {};          // 0: not configured on that device yet
     const int dev = launch_device();
@@ -960,9 +959,8 @@ cudaError_t nrc_gradients(NrcState& S, const float4* inputs, const float4* targe
     }
     cudaError_t e = cudaMemsetAsync(S.loss, 0, sizeof(float), st);
     // the forward stores the activations and the outputs of the batch
-    if(e == cudaSuccess) e = launch_forward<true, false, MRG_NRC_TRAIN_WARPS>(S, inputs, nullptr, nDevice, nMax, S.y, smCount, st);
-    const uint32_t tiles = (nMax + 16 * W - 1) / (16 * W);
-    const uint32_t grid = std::max(1u, std::min(tiles, (uint32_t)smCount * (uint32_t)perSM * 2u));
+    if(e == cudaSuccess) e = launch_forward<true, false>(S, inputs, nullptr, nDevice, nMax, S.y, smCount, st);
+    const uint32_t grid = std::max(1u, std::min((nMax + 15u) / 16u, (uint32_t)smCount * (uint32_t)perSM));
     if(e == cudaSuccess)
     {
         k_nrc_backward<W><<<grid, W * 32, bsmem, st>>>(S, inputs, S.y, targets, nDevice, nMax);

@@ -1,5 +1,5 @@
-"""Radiance-cache kernels at the edges of their tiles (16 samples a warp, 4 or
-32 warps a block, the small-query bound) against single samples: a sample's
+"""Radiance-cache kernels at the edges of their tiles (16 samples a warp, 32
+warps a block, partial rounds of blocks) against single samples: a sample's
 answer does not depend on its place in a batch."""
 import numpy as np
 import pytest
@@ -37,8 +37,8 @@ def _inputs(n, seed):
 def test_query_batches_agree(levels, log2):
     c = _cache(levels, log2)
     x = _inputs((1 << 17) + 33, 1)
-    whole = c.query(x)                                     # 32 warps a block, a partial round
-    # 4 warps a block up to 98,304 samples; 152 blocks of 32 warps hold 77,824
+    whole = c.query(x)                                     # a full round and a partial one
+    # 152 blocks of 32 warps hold 77,824 samples
     for n in (1, 15, 16, 17, 63, 64, 65, 1000, 77823, 77825, 98304, 98305, 1 << 17):
         assert torch.equal(c.query(x[:n].contiguous()), whole[:n]), n
     assert torch.equal(c.query(x[-40:].contiguous()), whole[-40:])
