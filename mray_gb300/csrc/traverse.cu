@@ -60,6 +60,7 @@ constexpr uint32_t kStepCap = 1u << 24;
 constexpr int kRefillMin = MRG_TRACE_REFILL;
 constexpr int kPostponeLanes = MRG_TRACE_POSTPONE;
 constexpr uint32_t kSpread = 2;
+constexpr uint32_t kFewRays = 4;
 
 struct LevelRay
 {
@@ -216,12 +217,13 @@ __device__ __forceinline__ uint32_t intersect_node(const WideNode* __restrict__ 
 // WT: the watertight triangle test on records that hold the three vertices.
 // ADD (with ANY): an unoccluded ray adds its radiance to its path (hits the
 // path radiance, meta the rays' radiance) instead of setting a visibility bit.
-// FEW: the cast has fewer rays than the grid has lanes.  A cast lasts as long
-// as its slowest warp, and a warp's pass costs its divergent lanes' paths one
-// after another, so the rays are spread: a warp keeps at most its share of
-// them (kSpread times it, at least one) in its first lanes and the rest idle.
-// The shares hold all rays, so nothing is claimed and no counter is cleared: an
-// atomic less in the chain of a ray (a 160x90 preview 170 -> 158 us).
+// FEW: the cast has few rays for the grid.  A warp's first rays are given to it
+// by its number, without a claim: an atomic less in the chain of a short cast
+// (a 160x90 preview 170 -> 158 us, the box scene's half million paths a pass
+// 791 -> 763 us a frame).  Below a ray a lane they are spread: a cast lasts as
+// long as its slowest warp, and a warp's pass costs its divergent lanes' paths
+// one after another, so a warp gets its share (kSpread times it, at least one)
+// in its first lanes and the rest idle.
 template<bool ANY, bool STATS, bool LOCAL = false, bool WT = false, bool ADD = false, bool FEW = false>
 __global__ void __launch_bounds__(kTraceTPB, MRG_TRACE_MIN_BLOCKS)
 k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
@@ -271,7 +273,7 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
     uint32_t statNodes = 0, statTris = 0, statInst = 0, statTlasNodes = 0, statDry = 0;
     uint32_t instHitBefore = kInvalidIndex;
     float instTBefore = 0.0f;
-    bool warpDone = false;
+    bool warpDone = false, started = false;
 
     uint32_t share = 32u;
     if(FEW)
@@ -293,9 +295,16 @@ k_trace(TraceScene sc, TraceScratch scr, float4* __restrict__ rays,
             uint32_t base = 0;
             if(FEW)
             {
-                // the warps' shares hold every ray: nothing to claim
-                base = ((blockIdx.x * kTraceTPB + threadIdx.x) >> 5) * share;
-                warpDone = true;
+                // the first rays by the warp's number, an atomic less to start with
+                const uint32_t given = gridDim.x * (kTraceTPB / 32) * share;
+                if(!started) base = ((blockIdx.x * kTraceTPB + threadIdx.x) >> 5) * share;
+                else
+                {
+                    if((int)lane == leader) base = atomicAdd(scr.workCounter, cnt);
+                    base = __shfl_sync(0xFFFFFFFFu, base, leader) + given;
+                }
+                started = true;
+                warpDone = base + cnt >= n || given >= n;
             }
             else
             {
@@ -585,9 +594,11 @@ cudaError_t clear_counter(const TraceScratch& scr, cudaStream_t st)
     return scr.cleared ? cudaSuccess : cudaMemsetAsync(scr.workCounter, 0, sizeof(uint32_t), st);
 }
 
-// A cast of n rays (with a device-side count: of at most n, 0: unknown).  FEW
-// while a warp's share stays below 32, some 68,000 rays: beyond that it only
-// costs registers (3.95M rays: 1.5%).  Closest hit on 27 x 82k triangles,
+// A cast of n rays (with a device-side count: of at most n, 0: unknown).  FEW up
+// to kFewRays a lane of the grid, some 545,000 rays: beyond that it only costs
+// registers (3.95M rays 1,700 -> 1,750 us in one kernel).  131,000 / 262,000 /
+// 524,000 rays on 27 x 82k triangles, closest hit 140 / 170 / 246 us without and
+// 139 / 168 / 242 with it.  Closest hit on 27 x 82k triangles,
 // 1,000 / 4,000 / 16,000 / 64,000 rays: 76 / 89 / 112 / 123 us filling the
 // warps, 56 / 70 / 90 / 124 spread; any hit 87 / 94 / 108 / 125 and 56 / 66 /
 // 93 / 122.  (Twice the even share: 1x and 4x gave 92 and 100 us at 16,000.
@@ -602,8 +613,14 @@ cudaError_t launch_cast(const TraceScene& sc, const TraceScratch& scr, const voi
     uint4* h = static_cast<uint4*>(hits);
     float2* m = static_cast<float2*>(meta);
     const int few = blocks_for<ANY, false, false, WT, ADD, true>(smCount);
-    if(n != 0u && n <= (uint32_t)few * kTraceTPB / kSpread)
+    const uint32_t lanes = (uint32_t)few * kTraceTPB;
+    if(n != 0u && n <= lanes * kFewRays)
     {
+        if(n > lanes)
+        {
+            cudaError_t e = clear_counter(scr, st);
+            if(e != cudaSuccess) return e;
+        }
         const uint32_t want = (n * kSpread + kTraceTPB / 32 - 1u) / (kTraceTPB / 32);
         k_trace<ANY, false, false, WT, ADD, true><<<std::min(want, (uint32_t)few), kTraceTPB, 0, st>>>(
             sc, scr, r, rayIdx, n, nDevice, h, m, visBits);

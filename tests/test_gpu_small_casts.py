@@ -7,7 +7,7 @@ from mray_gb300 import Accelerator, scenes
 
 pytestmark = pytest.mark.gpu
 
-LARGE = 160000         # above every limit of the small form
+LARGE = 600000         # above every limit of the small form
 
 
 def _soup(n, seed):
@@ -29,7 +29,7 @@ def test_small_casts_equal_large_ones(tris, ninst, watertight):
     for i in range(m.shape[0]):
         acc.add_instance(mesh, m[i], trans_key=i, accel_key=i)
     acc.construct()
-    rays = scenes.primary_rays(400, 400, 2, eye=(0, 0, -9), tan_half_fov=0.5)[:LARGE]
+    rays = scenes.primary_rays(800, 750, 2, eye=(0, 0, -9), tan_half_fov=0.5)[:LARGE]
     rng = np.random.default_rng(8)
     rays[::3, 0:3] = rng.uniform(-4, 4, rays[::3, 0:3].shape)    # origins inside the field
     rays[::7, 4:7] = np.eye(3)[rng.integers(0, 3, rays[::7].shape[0])] * rng.choice([-1.0, 1.0], (rays[::7].shape[0], 1))
@@ -48,7 +48,7 @@ def test_small_casts_equal_large_ones(tris, ninst, watertight):
     want = cast(rays)
     assert tris < 100 or (want[1][:, 0] != -1).sum() > 1000
     at = 0
-    for n in (1, 3, 31, 32, 33, 2127, 2129, 30000, 34047, 34049):
+    for n in (1, 3, 31, 32, 33, 2127, 2129, 30000, 34047, 34049, 136193, 250000):
         for a, b in zip(cast(rays[at:at + n]), want):
             np.testing.assert_array_equal(a.view(np.uint32), b[at:at + n].view(np.uint32))
         at += n
